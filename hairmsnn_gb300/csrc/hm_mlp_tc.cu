@@ -1504,100 +1504,152 @@ __global__ void __launch_bounds__(kTcThreads, 1) mlp_tc_bwd_kernel(const __grid_
   if (warp == 0) tmem_dealloc(tmem, p.ncols);
 }
 
-// ---- weight gradients of one layer: dW[o][i] = sum over rows dZ[row][o] h[row][i]
-// The batch is split in fixed chunks; a CTA accumulates its chunk in tensor
-// memory (A = dZ^T: the layer's outputs padded to 128 rows, B = h^T, K = the
-// 128 rows of a tile) and writes an FP32 partial [outputs][inputs].
-struct TcWgradArgs {
+// ---- weight gradients of every layer: dW[o][i] = sum over rows dZ[row][o] h[row][i]
+// One launch: blockIdx.y is a job (a layer's outputs x a tile of its
+// inputs), blockIdx.x a chunk of 2048 rows.  A CTA accumulates its chunk in
+// tensor memory (A = dZ^T, padded to 128 outputs, B = h^T, K = the rows) and
+// writes an FP32 partial; tc_wgrad_reduce_kernel sums the partials in chunk
+// order.  The tensor cores truncate when they accumulate, so the chunk fixes
+// the sums' last digits; what fills the GPU is the tile of inputs (see
+// tc_backward), which changes no bit.
+//
+// dZ and h lie row by row in memory, so both operands are read as MN-major
+// (the feature index contiguous): core matrices of 8 rows (k) x 8 features
+// (16 bytes per row), element (feature f, row k) of a stage at
+//   (f / 8) * kWgGroup + (k / 8) * 128 + (k % 8) * 16 + (f % 8) * 2.
+// A 16-byte piece of a row is copied as it is (cp.async), without the 2-byte
+// transposes a K-major operand needs.  A feature group is padded by 16 bytes
+// so that the pieces of one row fall into different banks.
+// Bound by the serial chain over a chunk (32 stages of 64 rows); a ring of
+// four stages keeps three stages' copies in flight under the MMAs.  A whole
+// FP16 step on 65,536 rows of the 5 x 64 network: 319 us; with a launch and a
+// reduction per layer, 32 CTAs each and 2-byte transposing stores, 958 us.
+constexpr int kWgRows = 64;                            // rows of a stage
+constexpr int kWgGroup = kWgRows / 8 * 128 + 16;       // bytes of one 8-feature group of a stage
+constexpr int kWgStages = 4;
+constexpr int kWgMaxJobs = 128;
+constexpr int64_t kWgChunk = 2048;                     // rows summed in tensor memory
+
+struct TcWgradJob {
   const uint16_t* dz;  // [n][dz_pitch], columns = outputs
-  int dz_pitch;
-  const uint16_t* h;   // [n][h_pitch], columns = inputs
+  const uint16_t* h;   // [n][h_pitch], from the job's first input column
   int h_pitch;
   int n_out, n_in;     // n_in: multiple of 16, <= 256
-  int64_t n;
-  int64_t chunk;
-  float* part;         // [splits][n_out][n_in]
+  int ld;              // row pitch of the layer's partial
+  int64_t part;        // the job's first element inside a chunk's partial
+};
+struct TcWgradArgs {
+  TcWgradJob job[kWgMaxJobs];
+  int dz_pitch;
+  int64_t n, chunk;
+  float* part;         // [chunks][part_stride]
+  int64_t part_stride;
   int* err;
-  int ncols;
+  int ncols, stage_bytes;
 };
 
+HM_D void cp_async16(uint32_t dst, const void* src, bool valid) {  // zero-fills when !valid
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(valid ? 16 : 0) : "memory");
+}
+HM_D void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int N>
+HM_D void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
+
 template <int PREC>
-__global__ void __launch_bounds__(kTcThreads, 1) mlp_tc_wgrad_kernel(const __grid_constant__ TcWgradArgs p) {
+__global__ void __launch_bounds__(kTcThreads) mlp_tc_wgrad_kernel(const __grid_constant__ TcWgradArgs p) {
   constexpr int FMT = PREC == TC_BF16 ? 1 : 0;
   extern __shared__ __align__(1024) uint8_t smem[];
-  uint8_t* A = smem;                        // [128 outputs][128 rows]
-  uint8_t* B = smem + kTcRows * kTcRows * 2;  // [n_in][128 rows]
-  uint64_t* bar = reinterpret_cast<uint64_t*>(B + (size_t)p.n_in * kTcRows * 2);
-  uint32_t* holder = reinterpret_cast<uint32_t*>(bar + 1);
+  __shared__ __align__(8) uint64_t bar[kWgStages];
+  __shared__ uint32_t holder;
+  const TcWgradJob& J = p.job[blockIdx.y];
   const int tid = threadIdx.x, warp = tid >> 5;
-  // A rows beyond the layer's outputs stay zero
-  for (int i = tid; i < kTcRows * kTcRows * 2 / 16; i += kTcThreads)
-    reinterpret_cast<uint4*>(A)[i] = make_uint4(0, 0, 0, 0);
+  const int ga = J.n_out / 8, gb = J.n_in / 8;  // 16-byte pieces of a row of dZ and of h
+  constexpr int kAGroups = kTcRows / 8;
+  // A's feature groups beyond the layer's outputs stay zero
+  for (int st = 0; st < kWgStages; ++st) {
+    uint4* z = reinterpret_cast<uint4*>(smem + st * p.stage_bytes + ga * kWgGroup);
+    for (int i = tid; i < (kAGroups - ga) * (kWgGroup / 16); i += kTcThreads) z[i] = make_uint4(0, 0, 0, 0);
+  }
   if (tid == 0) {
-    mbar_init(bar, 1);
+    for (int st = 0; st < kWgStages; ++st) mbar_init(bar + st, 1);
     fence_mbar_init();
   }
-  if (warp == 0) tmem_alloc(holder, p.ncols);
+  if (warp == 0) tmem_alloc(&holder, p.ncols);
   fence_proxy_async_smem();
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tmem = *holder;
-  const uint32_t a_base = smem_u32(A), b_base = smem_u32(B);
-  const uint32_t a_lbo = 16 * kTcRows, b_lbo = 16 * p.n_in;
-  uint32_t phase = 0;
-  bool failed = false;
+  const uint32_t tmem = holder;
+  const uint32_t s_base = smem_u32(smem);
   const int64_t r0 = blockIdx.x * p.chunk, r1 = min(p.n, r0 + p.chunk);
-  bool first = true;
-  for (int64_t t0 = r0; t0 < r1 && !failed; t0 += kTcRows) {
-    // transpose the tile's rows into A (dZ^T) and B (h^T): element (feature f,
-    // row k) at op_offset(rows_of_operand, f, 2k)
-    const int k = tid >> 1, hf = tid & 1;
-    const int64_t q = t0 + k;
-    const bool valid = q < r1;
-    for (int f = hf; f < p.n_out; f += 2) {
-      const uint16_t v = valid ? p.dz[q * p.dz_pitch + f] : (uint16_t)0;
-      *reinterpret_cast<uint16_t*>(A + op_offset(kTcRows, f, 2 * k)) = v;
+  const int iters = (int)((r1 - r0 + kWgRows - 1) / kWgRows);  // >= 1: the grid has no empty chunk
+  auto load = [&](int it) {
+    const uint32_t a = s_base + (uint32_t)((it % kWgStages) * p.stage_bytes), b = a + kAGroups * kWgGroup;
+    const int64_t q0 = r0 + (int64_t)it * kWgRows;
+    for (int i = tid; i < kWgRows * ga; i += kTcThreads) {
+      const int k = i / ga, g = i - k * ga;
+      const bool ok = q0 + k < r1;
+      cp_async16(a + g * kWgGroup + k * 16, J.dz + (ok ? q0 + k : r0) * p.dz_pitch + g * 8, ok);
     }
-    for (int f = hf; f < p.n_in; f += 2) {
-      const uint16_t v = valid ? p.h[q * p.h_pitch + f] : (uint16_t)0;
-      *reinterpret_cast<uint16_t*>(B + op_offset(p.n_in, f, 2 * k)) = v;
+    for (int i = tid; i < kWgRows * gb; i += kTcThreads) {
+      const int k = i / gb, g = i - k * gb;
+      const bool ok = q0 + k < r1;
+      cp_async16(b + g * kWgGroup + k * 16, J.h + (ok ? q0 + k : r0) * J.h_pitch + g * 8, ok);
     }
+  };
+  const uint32_t idesc = tc_idesc(kTcRows, J.n_in, FMT) | (1u << 15) | (1u << 16);  // A and B MN-major
+  bool failed = false;
+  // one cp.async group per step, empty past the end, so that the group to
+  // wait for is always the third newest
+  for (int it = 0; it < kWgStages - 1; ++it) {
+    if (it < iters) load(it);
+    cp_async_commit();
+  }
+  for (int it = 0; it < iters; ++it) {
+    const int st = it % kWgStages;
+    cp_async_wait<kWgStages - 2>();
     fence_proxy_async_smem();
     __syncthreads();
+    bool ok = true;
     if (tid == 0) {
       tc_fence_after();
-      const uint32_t idesc = tc_idesc(kTcRows, p.n_in, FMT);
-      for (int ks = 0; ks < kTcRows / 16; ++ks) {
-        const uint64_t ad = tc_sdesc(a_base + (uint32_t)ks * 2 * a_lbo, a_lbo, 128);
-        const uint64_t bd = tc_sdesc(b_base + (uint32_t)ks * 2 * b_lbo, b_lbo, 128);
-        tc_mma<false>(tmem, ad, bd, idesc, (!first || ks > 0) ? 1u : 0u);
-      }
-      tc_commit(bar);
+      const uint32_t a = s_base + (uint32_t)(st * p.stage_bytes), b = a + kAGroups * kWgGroup;
+      for (int ks = 0; ks < kWgRows / 16; ++ks)
+        tc_mma<false>(tmem, tc_sdesc(a + ks * 256, 128, kWgGroup), tc_sdesc(b + ks * 256, 128, kWgGroup), idesc,
+                      (it > 0 || ks > 0) ? 1u : 0u);
+      tc_commit(bar + st);
+      // the stage to refill was read by the MMAs of step it - 1
+      if (it >= 1) ok = mbar_wait_bounded(bar + (it - 1) % kWgStages, (uint32_t)(((it - 1) / kWgStages) & 1));
     }
-    // thread 0 (which committed) polls the barrier; the others sleep in the
-    // block barrier instead of spinning
-    const bool ok = threadIdx.x == 0 ? mbar_wait_bounded(bar, phase) : true;
-    phase ^= 1u;
-    if (__syncthreads_or(!ok)) failed = true;
-    tc_fence_after();
-    first = false;
+    if (__syncthreads_or(!ok)) {
+      failed = true;
+      break;
+    }
+    if (it + kWgStages - 1 < iters) load(it + kWgStages - 1);
+    cp_async_commit();
   }
-  // epilogue: row o of the accumulator (tensor-memory lane o) -> part
-  if (!failed && !first && warp < 4) {
-    const int o = tid;  // lanes 0..127 by warp quadrant
-    const uint32_t taddr = tmem + ((uint32_t)(warp * 32) << 16);
-    float* dst = p.part + ((int64_t)blockIdx.x * p.n_out + o) * p.n_in;
-    for (int c = 0; c < p.n_in; c += 16) {
+  if (!failed) {  // the last step's MMAs (a commit covers all earlier ones)
+    const int last = iters - 1;
+    const bool ok =
+        tid == 0 ? mbar_wait_bounded(bar + last % kWgStages, (uint32_t)((last / kWgStages) & 1)) : true;
+    failed = __syncthreads_or(!ok);
+  }
+  cp_async_wait<0>();
+  tc_fence_after();
+  // row o of the accumulator (tensor-memory lane o) -> the partial; the two
+  // halves of the block take alternate 16-column pieces
+  if (!failed) {
+    const int o = (warp & 3) * 32 + (tid & 31);
+    const uint32_t taddr = tmem + ((uint32_t)((warp & 3) * 32) << 16);
+    float* dst = p.part + blockIdx.x * p.part_stride + J.part + (int64_t)o * J.ld;
+    for (int c = (warp >> 2) * 16; c < J.n_in; c += 32) {
       float t[16];
       tmem_ld16(taddr + c, t);
-      if (o < p.n_out)
+      if (o < J.n_out)
 #pragma unroll
-        for (int e = 0; e < 16; ++e) dst[c + e] = t[e];
+        for (int e = 0; e < 16; e += 4)
+          *reinterpret_cast<float4*>(dst + c + e) = make_float4(t[e], t[e + 1], t[e + 2], t[e + 3]);
     }
-  } else if (!failed && first && warp < 4 && tid < p.n_out) {
-    float* dst = p.part + ((int64_t)blockIdx.x * p.n_out + tid) * p.n_in;
-    for (int c = 0; c < p.n_in; ++c) dst[c] = 0.f;
   }
   if (failed && tid == 0) atomicOr(p.err, 1);
   tc_fence_before();
@@ -1606,26 +1658,29 @@ __global__ void __launch_bounds__(kTcThreads, 1) mlp_tc_wgrad_kernel(const __gri
   if (warp == 0) tmem_dealloc(tmem, p.ncols);
 }
 
-__global__ void tc_reduce_kernel(const float* __restrict__ part, int splits, int64_t mn, float* __restrict__ out) {
-  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < mn; i += (int64_t)gridDim.x * blockDim.x) {
-    float s = 0.f;
-    for (int k = 0; k < splits; ++k) s += part[(int64_t)k * mn + i];
-    out[i] = s;
-  }
-}
-
-// The same for a layer whose K is padded past its fan-in (E4M3 layer 0):
-// partial rows are K wide, the parameter rows fan_in wide.
-__global__ void tc_reduce_pad_kernel(const float* __restrict__ part, int splits, int N, int K, int fan_in,
-                                     float* __restrict__ out) {
-  const int64_t mn = (int64_t)N * K;
-  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < (int64_t)N * fan_in;
-       i += (int64_t)gridDim.x * blockDim.x) {
-    const int64_t src = (i / fan_in) * K + i % fan_in;
-    float s = 0.f;
-    for (int k = 0; k < splits; ++k) s += part[(int64_t)k * mn + src];
-    out[i] = s;
-  }
+// Sums the chunks' partials in chunk order into the matrix gradients of
+// every layer.  A partial's rows are K[l] wide, the parameters' fan_in wide
+// (they differ in the E4M3 layer 0, whose K is padded).
+struct TcReduceArgs {
+  int n_layers;
+  int64_t goff[16];  // first gradient of each layer; [n_layers]: their number
+  int64_t poff[16];  // first element of each layer inside a partial
+  int fan_in[16], ld[16];
+  int64_t stride;
+  int chunks;
+};
+__global__ void __launch_bounds__(128) tc_wgrad_reduce_kernel(const __grid_constant__ TcReduceArgs p,
+                                                              const float* __restrict__ part, float* __restrict__ out) {
+  const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  if (i >= p.goff[p.n_layers]) return;
+  int l = 0;
+  while (l + 1 < p.n_layers && i >= p.goff[l + 1]) ++l;
+  const int64_t j = i - p.goff[l];
+  const float* src = part + p.poff[l] + (j / p.fan_in[l]) * p.ld[l] + j % p.fan_in[l];
+  float s = 0.f;
+#pragma unroll 8
+  for (int k = 0; k < p.chunks; ++k) s += __ldg(src + k * p.stride);
+  out[i] = s;
 }
 
 __global__ void tc_loss_reduce_kernel(const float* __restrict__ part, int nb, float* __restrict__ out) {
@@ -1700,54 +1755,79 @@ int tc_backward(const MlpDims& d, const TcPack& pk, const TcTrainBufs& b, const 
   if (s) return s;
   tc_loss_reduce_kernel<<<1, 32, 0, st>>>(b.loss_part, blocks, loss_out);
   HM_CHECK_LAUNCH("tc_loss_reduce_kernel");
-  // weight gradients
-  const int64_t chunk = 2048;
-  const int splits = (int)((n + chunk - 1) / chunk);
-  int64_t need = 0;
-  for (int l = 0; l <= L; ++l) need = std::max<int64_t>(need, (int64_t)splits * pk.N[l] * pk.K[l]);
+  // weight gradients: jobs of one layer x a tile of its inputs.  64 inputs
+  // per tile; 32 while that still gives at most one CTA per SM.  A whole
+  // step, FP16, tiles of 256 / 128 / 64 / 32 inputs: 5 x 64 network, 65,536
+  // rows 339 / 333 / 319 / 354 us, 16,384 rows 240 / 226 / 219 / 213 us;
+  // 5 x 128, 16,384 rows 292 / 275 / 267 / 285 us.
+  int dev = 0, sms = 0;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  const int chunks = (int)((n + kWgChunk - 1) / kWgChunk);
+  auto count_jobs = [&](int t) {
+    int c = 0;
+    for (int l = 0; l <= L; ++l) c += (pk.K[l] + t - 1) / t;
+    return c;
+  };
+  int tile = chunks * (int64_t)count_jobs(32) <= sms ? 32 : 64;
+  while (count_jobs(tile) > kWgMaxJobs && tile < 256) tile *= 2;
+  TcWgradArgs g;
+  memset(&g, 0, sizeof(g));
+  TcReduceArgs r{};
+  const int wz = std::max(W, 16);
+  int jobs = 0, max_in = 0;
+  int64_t poff = 0;
+  for (int l = 0; l <= L; ++l) {
+    const int N = pk.N[l], K = pk.K[l];
+    for (int c = 0; c < K; c += tile) {
+      if (jobs == kWgMaxJobs) return hm_set_error("mlp: too many weight-gradient tiles"), HM_EUNSUPPORTED;
+      TcWgradJob& j = g.job[jobs++];
+      j.dz = b.dz16 + (int64_t)l * n * wz;
+      j.h = (l == 0 ? b.x16 : b.h16 + (int64_t)(l - 1) * n * W) + c;
+      j.h_pitch = l == 0 ? K : W;
+      j.n_out = N;
+      j.n_in = std::min(tile, K - c);
+      j.ld = K;
+      j.part = poff + c;
+      max_in = std::max(max_in, j.n_in);
+    }
+    // the layer's weights are [out][fan_in] with fan_in <= K[l]
+    r.goff[l] = d.layer_off[l];
+    r.poff[l] = poff;
+    r.fan_in[l] = l == 0 ? d.in_pad : W;
+    r.ld[l] = K;
+    poff += (int64_t)N * K;
+  }
+  r.n_layers = L + 1;
+  r.goff[L + 1] = d.n_net_params;
+  r.stride = poff;
+  r.chunks = chunks;
+  const int64_t need = (int64_t)chunks * poff;
   if (need > *dw_cap) {
     cudaFree(*dw_part);
     *dw_part = nullptr;
+    *dw_cap = 0;
     cudaError_t e = cudaMalloc(dw_part, need * sizeof(float));
     if (e != cudaSuccess) return hm_cuda_status(e, "tensor-core dW partials");
     *dw_cap = need;
   }
-  for (int l = 0; l <= L; ++l) {
-    TcWgradArgs g;
-    g.n_out = pk.N[l];
-    g.n_in = pk.K[l];
-    g.dz = b.dz16 + (int64_t)l * n * std::max(W, 16);
-    g.dz_pitch = std::max(W, 16);
-    g.h = l == 0 ? b.x16 : b.h16 + (int64_t)(l - 1) * n * W;
-    g.h_pitch = l == 0 ? pk.K[0] : W;
-    g.n = n;
-    g.chunk = chunk;
-    g.part = *dw_part;
-    g.err = err_flag;
-    int nc = 32;
-    while (nc < g.n_in) nc *= 2;
-    g.ncols = nc;
-    const size_t sm = (size_t)kTcRows * kTcRows * 2 + (size_t)g.n_in * kTcRows * 2 + 64;
-    if (pk.precision == HM_PREC_BF16) {
-      cudaFuncSetAttribute(mlp_tc_wgrad_kernel<TC_BF16>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-      mlp_tc_wgrad_kernel<TC_BF16><<<splits, kTcThreads, sm, st>>>(g);
-    } else {
-      cudaFuncSetAttribute(mlp_tc_wgrad_kernel<TC_FP16>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-      mlp_tc_wgrad_kernel<TC_FP16><<<splits, kTcThreads, sm, st>>>(g);
-    }
-    HM_CHECK_LAUNCH("mlp_tc_wgrad_kernel");
-    // the layer's weights are [out][in_l] with in_l = fan_in (<= K[l]); the
-    // partial rows are K[l] wide, the parameters fan_in wide
-    const int fan_in = l == 0 ? d.in_pad : W;
-    const int64_t mn = (int64_t)pk.N[l] * pk.K[l];
-    if (fan_in == pk.K[l]) {
-      tc_reduce_kernel<<<256, 256, 0, st>>>(*dw_part, splits, mn, grads + d.layer_off[l]);
-      HM_CHECK_LAUNCH("tc_reduce_kernel");
-    } else {
-      tc_reduce_pad_kernel<<<256, 256, 0, st>>>(*dw_part, splits, pk.N[l], pk.K[l], fan_in, grads + d.layer_off[l]);
-      HM_CHECK_LAUNCH("tc_reduce_pad_kernel");
-    }
-  }
+  g.dz_pitch = wz;
+  g.n = n;
+  g.chunk = kWgChunk;
+  g.part = *dw_part;
+  g.part_stride = poff;
+  g.err = err_flag;
+  g.ncols = 32;
+  while (g.ncols < max_in) g.ncols *= 2;
+  g.stage_bytes = (kTcRows / 8 + max_in / 8) * kWgGroup;
+  const size_t sm = (size_t)kWgStages * g.stage_bytes;
+  auto kern = pk.precision == HM_PREC_BF16 ? mlp_tc_wgrad_kernel<TC_BF16> : mlp_tc_wgrad_kernel<TC_FP16>;
+  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+  if (e != cudaSuccess) return hm_cuda_status(e, "mlp_tc_wgrad_kernel smem");
+  kern<<<dim3((unsigned)chunks, (unsigned)jobs), kTcThreads, sm, st>>>(g);
+  HM_CHECK_LAUNCH("mlp_tc_wgrad_kernel");
+  tc_wgrad_reduce_kernel<<<(unsigned)((d.n_net_params + 127) / 128), 128, 0, st>>>(r, *dw_part, grads);
+  HM_CHECK_LAUNCH("tc_wgrad_reduce_kernel");
   return HM_OK;
 }
 
