@@ -137,6 +137,27 @@ HM_D void loss_grad(int loss, const float* pred, const float* tgt, int out_ch, f
   *value = v;
 }
 
+// 16-byte asynchronous copies global -> shared
+HM_D void cp_async16(uint32_t dst, const void* src, bool valid) {  // zero-fills when !valid
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(valid ? 16 : 0) : "memory");
+}
+HM_D void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int N>
+HM_D void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
+
+// ---- sums of the weight-gradient partials (one per chunk of the batch)
+struct WgradSum {
+  int n_layers, chunks;
+  int64_t goff[16];  // first gradient of each layer; [n_layers]: their number
+  int64_t poff[16];  // first element of each layer inside a partial
+  int fan_in[16], ld[16];  // row length of the parameters and of the partial
+  int64_t stride;          // elements of a partial
+};
+// grads = the partials' sums in chunk order, *loss_out = the sum of n_loss
+// partial losses.
+int wgrad_sum(const WgradSum& r, const float* part, float* grads, const float* loss_part, int n_loss, float* loss_out,
+              cudaStream_t st);
+
 // ---- tensor-core (tcgen05) forward for HM_PREC_FP16 / BF16 / FP8_E4M3
 // Weights are repacked from the FP32 master copy into the operand layout of
 // the MMA (K-major, 8-row x 16-byte core matrices) whenever they change.

@@ -1508,7 +1508,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) mlp_tc_bwd_kernel(const __grid_
 // One launch: blockIdx.y is a job (a layer's outputs x a tile of its
 // inputs), blockIdx.x a chunk of 2048 rows.  A CTA accumulates its chunk in
 // tensor memory (A = dZ^T, padded to 128 outputs, B = h^T, K = the rows) and
-// writes an FP32 partial; tc_wgrad_reduce_kernel sums the partials in chunk
+// writes an FP32 partial; wgrad_sum_kernel sums the partials in chunk
 // order.  The tensor cores truncate when they accumulate, so the chunk fixes
 // the sums' last digits; what fills the GPU is the tile of inputs (see
 // tc_backward), which changes no bit.
@@ -1547,13 +1547,6 @@ struct TcWgradArgs {
   int* err;
   int ncols, stage_bytes;
 };
-
-HM_D void cp_async16(uint32_t dst, const void* src, bool valid) {  // zero-fills when !valid
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(valid ? 16 : 0) : "memory");
-}
-HM_D void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-template <int N>
-HM_D void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
 
 template <int PREC>
 __global__ void __launch_bounds__(kTcThreads) mlp_tc_wgrad_kernel(const __grid_constant__ TcWgradArgs p) {
@@ -1659,18 +1652,28 @@ __global__ void __launch_bounds__(kTcThreads) mlp_tc_wgrad_kernel(const __grid_c
 }
 
 // Sums the chunks' partials in chunk order into the matrix gradients of
-// every layer.  A partial's rows are K[l] wide, the parameters' fan_in wide
-// (they differ in the E4M3 layer 0, whose K is padded).
-struct TcReduceArgs {
-  int n_layers;
-  int64_t goff[16];  // first gradient of each layer; [n_layers]: their number
-  int64_t poff[16];  // first element of each layer inside a partial
-  int fan_in[16], ld[16];
-  int64_t stride;
-  int chunks;
-};
-__global__ void __launch_bounds__(128) tc_wgrad_reduce_kernel(const __grid_constant__ TcReduceArgs p,
-                                                              const float* __restrict__ part, float* __restrict__ out) {
+// every layer.  A partial's rows are ld[l] wide, the parameters' fan_in wide
+// (they differ in the E4M3 layer 0, whose K is padded).  One block more than
+// the gradients need sums the blocks' losses, in block order (a launch of one
+// thread reading them from memory took 6 us).
+__global__ void __launch_bounds__(128) wgrad_sum_kernel(const __grid_constant__ WgradSum p,
+                                                        const float* __restrict__ part, float* __restrict__ out,
+                                                        const float* __restrict__ loss_part, int n_loss,
+                                                        float* __restrict__ loss_out) {
+  if (blockIdx.x == gridDim.x - 1) {
+    __shared__ float v[1024];
+    float s = 0.f;
+    for (int base = 0; base < n_loss; base += 1024) {
+      const int m = min(1024, n_loss - base);
+      for (int i = threadIdx.x; i < m; i += 128) v[i] = loss_part[base + i];
+      __syncthreads();
+      if (threadIdx.x == 0)
+        for (int i = 0; i < m; ++i) s += v[i];
+      __syncthreads();
+    }
+    if (threadIdx.x == 0) *loss_out = s;
+    return;
+  }
   const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (i >= p.goff[p.n_layers]) return;
   int l = 0;
@@ -1678,17 +1681,17 @@ __global__ void __launch_bounds__(128) tc_wgrad_reduce_kernel(const __grid_const
   const int64_t j = i - p.goff[l];
   const float* src = part + p.poff[l] + (j / p.fan_in[l]) * p.ld[l] + j % p.fan_in[l];
   float s = 0.f;
-#pragma unroll 8
+#pragma unroll 16
   for (int k = 0; k < p.chunks; ++k) s += __ldg(src + k * p.stride);
   out[i] = s;
 }
 
-__global__ void tc_loss_reduce_kernel(const float* __restrict__ part, int nb, float* __restrict__ out) {
-  if (threadIdx.x == 0 && blockIdx.x == 0) {
-    float s = 0.f;
-    for (int i = 0; i < nb; ++i) s += part[i];
-    *out = s;
-  }
+int wgrad_sum(const WgradSum& r, const float* part, float* grads, const float* loss_part, int n_loss, float* loss_out,
+              cudaStream_t st) {
+  wgrad_sum_kernel<<<(unsigned)((r.goff[r.n_layers] + 127) / 128 + 1), 128, 0, st>>>(r, part, grads, loss_part, n_loss,
+                                                                                    loss_out);
+  HM_CHECK_LAUNCH("wgrad_sum_kernel");
+  return HM_OK;
 }
 
 template <int PREC, int W>
@@ -1753,8 +1756,6 @@ int tc_backward(const MlpDims& d, const TcPack& pk, const TcTrainBufs& b, const 
     s = W == 16 ? tc_bwd_launch<TC_FP16, 16>(a, smem, st, &blocks) : W == 32 ? tc_bwd_launch<TC_FP16, 32>(a, smem, st, &blocks)
         : W == 64 ? tc_bwd_launch<TC_FP16, 64>(a, smem, st, &blocks) : tc_bwd_launch<TC_FP16, 128>(a, smem, st, &blocks);
   if (s) return s;
-  tc_loss_reduce_kernel<<<1, 32, 0, st>>>(b.loss_part, blocks, loss_out);
-  HM_CHECK_LAUNCH("tc_loss_reduce_kernel");
   // weight gradients: jobs of one layer x a tile of its inputs.  64 inputs
   // per tile; 32 while that still gives at most one CTA per SM.  A whole
   // step, FP16, tiles of 256 / 128 / 64 / 32 inputs: 5 x 64 network, 65,536
@@ -1773,7 +1774,7 @@ int tc_backward(const MlpDims& d, const TcPack& pk, const TcTrainBufs& b, const 
   while (count_jobs(tile) > kWgMaxJobs && tile < 256) tile *= 2;
   TcWgradArgs g;
   memset(&g, 0, sizeof(g));
-  TcReduceArgs r{};
+  WgradSum r{};
   const int wz = std::max(W, 16);
   int jobs = 0, max_in = 0;
   int64_t poff = 0;
@@ -1826,9 +1827,7 @@ int tc_backward(const MlpDims& d, const TcPack& pk, const TcTrainBufs& b, const 
   if (e != cudaSuccess) return hm_cuda_status(e, "mlp_tc_wgrad_kernel smem");
   kern<<<dim3((unsigned)chunks, (unsigned)jobs), kTcThreads, sm, st>>>(g);
   HM_CHECK_LAUNCH("mlp_tc_wgrad_kernel");
-  tc_wgrad_reduce_kernel<<<(unsigned)((d.n_net_params + 127) / 128), 128, 0, st>>>(r, *dw_part, grads);
-  HM_CHECK_LAUNCH("tc_wgrad_reduce_kernel");
-  return HM_OK;
+  return wgrad_sum(r, *dw_part, grads, b.loss_part, blocks, loss_out, st);
 }
 
 // ---- the bounded wait's expiry, exercised on purpose (tests)
