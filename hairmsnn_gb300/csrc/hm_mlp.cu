@@ -224,9 +224,7 @@ HM_D void grid_level(const EncSeg& s, int l, const float* __restrict__ table, fl
   const float wx = fx - gx, wy = fy - gy, wz = fz - gz;
   const uint32_t ix = (uint32_t)(int)gx, iy = (uint32_t)(int)gy, iz = (uint32_t)(int)gz;
   uint32_t e[8];
-#pragma unroll
-  for (int c = 0; c < 8; ++c)
-    e[c] = s.level_off[l] + grid_index(s, l, ix + (c & 1), iy + ((c >> 1) & 1), iz + ((c >> 2) & 1));
+  grid_entries(s, l, ix, iy, iz, e);
   auto weight = [&](int c) {
     return ((c & 1) ? wx : 1.f - wx) * (((c >> 1) & 1) ? wy : 1.f - wy) * (((c >> 2) & 1) ? wz : 1.f - wz);
   };
@@ -279,7 +277,7 @@ __global__ void __launch_bounds__(kEncThreads) encode_kernel(const __grid_consta
       units = s.n_dims * s.n_freq;
       for (int k = warp; k < units; k += kWarps) {
         const int dim = k / s.n_freq;
-        const float a = ldexpf(xin[s.in_off + dim], k - dim * s.n_freq) * kPi;
+        const float a = scale_pow2(xin[s.in_off + dim], k - dim * s.n_freq) * kPi;
         o[2 * k] = sinf(a);
         o[2 * k + 1] = sinf(a + 0.5f * kPi);
       }
@@ -343,16 +341,16 @@ __global__ void __launch_bounds__(256) grid_bwd_kernel(const __grid_constant__ E
   const float gx = floorf(fx), gy = floorf(fy), gz = floorf(fz);
   const float wx = fx - gx, wy = fy - gy, wz = fz - gz;
   const uint32_t ix = (uint32_t)(int)gx, iy = (uint32_t)(int)gy, iz = (uint32_t)(int)gz;
+  uint32_t e[8];
+  grid_entries(s, l, ix, iy, iz, e);
   for (int f = 0; f < s.n_feat; ++f) {
     const float gv = g[f];
     if (gv == 0.f) continue;
 #pragma unroll
     for (int c = 0; c < 8; ++c) {
-      const uint32_t cx = ix + (c & 1), cy = iy + ((c >> 1) & 1), cz = iz + ((c >> 2) & 1);
       const float w = ((c & 1) ? wx : 1.f - wx) * (((c >> 1) & 1) ? wy : 1.f - wy) * (((c >> 2) & 1) ? wz : 1.f - wz);
       const long long v = __float2ll_rn(w * gv * kGridFix);
-      const uint32_t e = s.level_off[l] + grid_index(s, l, cx, cy, cz);
-      if (v != 0) atomicAdd((unsigned long long*)(tg + (int64_t)e * s.n_feat + f), (unsigned long long)v);
+      if (v != 0) atomicAdd((unsigned long long*)(tg + (int64_t)e[c] * s.n_feat + f), (unsigned long long)v);
     }
   }
 }

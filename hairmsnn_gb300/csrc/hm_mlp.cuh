@@ -96,22 +96,35 @@ HM_D float oneblob_cdf(float boundary, float x, float nb) {
          quartic_cdf(boundary - x + 1.0f, nb);
 }
 
-HM_D uint32_t grid_index(const EncSeg& s, int l, uint32_t x, uint32_t y, uint32_t z) {
-  const uint32_t size = s.level_size[l], res = s.level_res[l];
-  uint32_t stride = 1, index = 0;
-  index += x * stride;
-  stride *= res;
-  if (stride <= size) {
-    index += y * stride;
-    stride *= res;
-    if (stride <= size) {
-      index += z * stride;
-      stride *= res;
-    }
+// Table entries of the eight corners of the cell (x, y, z) of level l (corner
+// c: +1 along axis a where bit a of c is set): dense index while the grid fits
+// the table, else the spatial hash.  The level's form is decided once for all
+// corners, so that their loads can follow one another; hashed levels have 2^T
+// entries and need no division.
+HM_D void grid_entries(const EncSeg& s, int l, uint32_t x, uint32_t y, uint32_t z, uint32_t (&e)[8]) {
+  const uint32_t size = s.level_size[l], s1 = s.level_res[l], s2 = s1 * s1, s3 = s2 * s1, off = s.level_off[l];
+  if (s1 > size || s2 > size || s3 > size) {
+    const uint32_t py = 2654435761u, pz = 805459861u;
+    const uint32_t hy[2] = {y * py, y * py + py}, hz[2] = {z * pz, z * pz + pz};
+#pragma unroll
+    for (int c = 0; c < 8; ++c) e[c] = (x + (c & 1)) ^ hy[(c >> 1) & 1] ^ hz[(c >> 2) & 1];
+  } else {
+    const uint32_t i = x + y * s1 + z * s2;
+#pragma unroll
+    for (int c = 0; c < 8; ++c) e[c] = i + (c & 1) + ((c >> 1) & 1) * s1 + ((c >> 2) & 1) * s2;
   }
-  if (size < stride) index = (x * 1u) ^ (y * 2654435761u) ^ (z * 805459861u);
-  return index % size;
+  if ((size & (size - 1)) == 0) {
+#pragma unroll
+    for (int c = 0; c < 8; ++c) e[c] = off + (e[c] & (size - 1));
+  } else {
+#pragma unroll
+    for (int c = 0; c < 8; ++c) e[c] = off + e[c] % size;
+  }
 }
+
+// 2^f x for f >= 0: the same value as ldexpf (the product of a float and a
+// power of two is exact or overflows), without its range handling.
+HM_D float scale_pow2(float x, int f) { return f < 128 ? x * __int_as_float((127 + f) << 23) : ldexpf(x, f); }
 
 
 // Loss gradient of one query (tcnn semantics, averaged over n * out_ch).
@@ -202,8 +215,8 @@ void tc_pack_free(TcPack* pk);
 // encoder warps and layer warps overlapped in one CTA per SM, no
 // workspace); with a workspace of at least tc_encode_bytes, the encode
 // kernel and then the layer kernel loading its input tiles by bulk copies
-// (networks with a hash grid, E4M3, width 128); without one, the layer
-// kernel encoding its own tiles.
+// (E4M3, width 16 / 128, wide encodings); without one, the layer kernel
+// encoding its own tiles.
 int64_t tc_encode_bytes(const MlpDims& d, const TcPack& pk, int64_t n);
 // Whether tc_forward would use a workspace (false where the warp-specialised
 // kernel runs: no encoded operands in device memory).

@@ -271,7 +271,7 @@ HM_D void enc_range(const MlpDims& d, const float* __restrict__ xin, const float
       int dim = u / s.n_freq, f = u - dim * s.n_freq;
       for (int j = j0; j < j1;) {
         float sn, cs;
-        sincospif(ldexpf(xin[s.in_off + dim], f), &sn, &cs);
+        sincospif(scale_pow2(xin[s.in_off + dim], f), &sn, &cs);
         if (!(j & 1) && j + 1 < j1) {
           pk.push2(sn, cs);
           j += 2;
@@ -368,17 +368,15 @@ HM_D void enc_range(const MlpDims& d, const float* __restrict__ xin, const float
         float acc[8];
 #pragma unroll
         for (int q = 0; q < 8; ++q) acc[q] = 0.f;
+        uint32_t e[8];
+        grid_entries(s, l, ix, iy, iz, e);
         if (pair_table) {
           // two features per entry: the eight corners' entries are loaded
           // first (eight 8-byte gathers in flight), then accumulated in
           // corner order as below
           float2 tv[8];
 #pragma unroll
-          for (int c = 0; c < 8; ++c) {
-            const uint32_t cx = ix + (c & 1), cy = iy + ((c >> 1) & 1), cz = iz + ((c >> 2) & 1);
-            const uint32_t e = s.level_off[l] + grid_index(s, l, cx, cy, cz);
-            tv[c] = __ldg(reinterpret_cast<const float2*>(table) + e);
-          }
+          for (int c = 0; c < 8; ++c) tv[c] = __ldg(reinterpret_cast<const float2*>(table) + e[c]);
 #pragma unroll
           for (int c = 0; c < 8; ++c) {
             const float w = ((c & 1) ? wx : 1.f - wx) * (((c >> 1) & 1) ? wy : 1.f - wy) *
@@ -387,12 +385,11 @@ HM_D void enc_range(const MlpDims& d, const float* __restrict__ xin, const float
             acc[1] += w * tv[c].y;
           }
         } else {
+#pragma unroll
           for (int c = 0; c < 8; ++c) {
-            const uint32_t cx = ix + (c & 1), cy = iy + ((c >> 1) & 1), cz = iz + ((c >> 2) & 1);
             const float w = ((c & 1) ? wx : 1.f - wx) * (((c >> 1) & 1) ? wy : 1.f - wy) *
                             (((c >> 2) & 1) ? wz : 1.f - wz);
-            const uint32_t e = s.level_off[l] + grid_index(s, l, cx, cy, cz);
-            const float* tv = table + (int64_t)e * s.n_feat;
+            const float* tv = table + (int64_t)e[c] * s.n_feat;
 #pragma unroll
             for (int q = 0; q < 8; ++q)
               if (q < s.n_feat) acc[q] += w * __ldg(tv + q);
@@ -423,6 +420,236 @@ HM_D void enc_range(const MlpDims& d, const float* __restrict__ xin, const float
   int k = max(kb, d.n_enc);
   for (; k + 1 < ke; k += 2) pk.push2(k < d.in_pad ? 1.f : 0.f, k + 1 < d.in_pad ? 1.f : 0.f);
   if (k < ke) pk.push(k < d.in_pad ? 1.f : 0.f);
+}
+
+// ---- encodings whose segments are made of whole 8-feature units
+// (enc_units_ok): every Frequency, OneBlob and hash-grid segment starts and
+// ends on a multiple of 8 features, and what follows the last one is identity
+// inputs and padding.  The same values as enc_range, built a unit at a time
+// in registers and stored to the unit's address: no packing register, no
+// per-feature bookkeeping.  A OneBlob input's bins are all zero but five
+// consecutive ones (circularly): its units are stored as zeros and the two or
+// three words that hold the five masses are stored over them, where the
+// mass-by-mass selection cost about eleven instructions per bin.
+// The kernels that encode are bound by instruction issue (31 per sincospif, 27
+// per OneBlob edge).  Feature by feature through the packing register of
+// enc_range -> by units: tc_encode_kernel<E4M3>, 300,007 queries of the 5 x 128
+// network 104 -> 41 us; mlp_tc_fused_kernel<FP16, 64>, 2^20 queries 498 -> 248
+// us (about 5000 instructions per query, 12,000 before).
+//
+// The caller's row: operand bytes of feature k at
+//   a + (k * bytes / 16) * 2048 + k * bytes % 16    (128-row core-matrix layout)
+// and, in a training forward, copies of it for the backward pass: `mirror`
+// (16-bit operands as they are) or `mirror16` (FP16 of an E4M3 row's unscaled
+// features), with unit u at + u * mirror_unit bytes.
+struct EncRow {
+  uint8_t* a;
+  uint8_t* mirror;
+  uint32_t mirror_unit;
+  float scale;
+};
+
+HM_HD bool enc_units_ok(const MlpDims& d) {
+  for (int si = 0; si < d.n_segs; ++si) {
+    const EncSeg& s = d.segs[si];
+    if (s.out_off % 8 != 0) return false;
+    if (s.type == ENC_IDENTITY) return si == d.n_segs - 1;
+    if (s.n_out % 8 != 0) return false;
+    if (s.type == ENC_FREQUENCY && s.n_freq > 120) return false;
+    if (s.type == ENC_ONEBLOB && s.n_bins % 8 != 0 && s.n_bins != 4) return false;
+    if (s.type == ENC_HASHGRID && s.n_feat != 2) return false;
+  }
+  return true;
+}
+
+template <int PREC>
+HM_D void enc_store8(const EncRow& r, int k, const float (&v)[8]) {
+  if (PREC == TC_E4M3) {
+    if (r.mirror) {
+      uint4 h;
+      h.x = pack2<TC_FP16>(v[0], v[1]);
+      h.y = pack2<TC_FP16>(v[2], v[3]);
+      h.z = pack2<TC_FP16>(v[4], v[5]);
+      h.w = pack2<TC_FP16>(v[6], v[7]);
+      *reinterpret_cast<uint4*>(r.mirror + (uint32_t)(k >> 3) * r.mirror_unit) = h;
+    }
+    uint2 w;
+    w.x = pack4_e4m3(v[0] * r.scale, v[1] * r.scale, v[2] * r.scale, v[3] * r.scale);
+    w.y = pack4_e4m3(v[4] * r.scale, v[5] * r.scale, v[6] * r.scale, v[7] * r.scale);
+    *reinterpret_cast<uint2*>(r.a + (uint32_t)(k >> 4) * 2048u + (uint32_t)(k & 8)) = w;
+  } else {
+    constexpr int P16 = PREC == TC_E4M3 ? TC_FP16 : PREC;
+    uint4 w;
+    w.x = pack2<P16>(v[0], v[1]);
+    w.y = pack2<P16>(v[2], v[3]);
+    w.z = pack2<P16>(v[4], v[5]);
+    w.w = pack2<P16>(v[6], v[7]);
+    *reinterpret_cast<uint4*>(r.a + (uint32_t)(k >> 3) * 2048u) = w;
+    if (r.mirror) *reinterpret_cast<uint4*>(r.mirror + (uint32_t)(k >> 3) * r.mirror_unit) = w;
+  }
+}
+
+// The masses m of bins first .. first + 4 (mod n_bins) of the OneBlob input
+// whose features start at k0, as the words that hold them; only words of
+// features [lo, hi) (multiples of 8) are stored.
+template <int PREC>
+HM_D void enc_store_window(const EncRow& r, int k0, int n_bins, int first, const float (&m)[5], int lo, int hi) {
+  if (PREC == TC_E4M3) {  // four lanes per word, two words
+    const uint64_t b = (uint64_t)pack4_e4m3(m[0] * r.scale, m[1] * r.scale, m[2] * r.scale, m[3] * r.scale) |
+                       (uint64_t)(pack4_e4m3(m[4] * r.scale, 0.f, 0.f, 0.f) & 0xFFu) << 32;
+    const uint64_t v = b << (8 * (first & 3));
+    int w = first & ~3;
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+      const int k = k0 + w;
+      if (k >= lo && k < hi)
+        *reinterpret_cast<uint32_t*>(r.a + (uint32_t)(k >> 4) * 2048u + (uint32_t)(k & 15)) =
+            i ? (uint32_t)(v >> 32) : (uint32_t)v;
+      w += 4;
+      w -= w >= n_bins ? n_bins : 0;
+    }
+    if (!r.mirror) return;
+  }
+  constexpr int P16 = PREC == TC_E4M3 ? TC_FP16 : PREC;
+  const bool odd = first & 1;
+  const uint32_t v[3] = {odd ? pack2<P16>(0.f, m[0]) : pack2<P16>(m[0], m[1]),
+                         odd ? pack2<P16>(m[1], m[2]) : pack2<P16>(m[2], m[3]),
+                         odd ? pack2<P16>(m[3], m[4]) : pack2<P16>(m[4], 0.f)};
+  int w = first & ~1;
+#pragma unroll
+  for (int i = 0; i < 3; ++i) {
+    const int k = k0 + w;
+    if (k >= lo && k < hi) {
+      const uint32_t u = (uint32_t)(k >> 3), byte = (uint32_t)(k & 7) * 2u;
+      if (PREC != TC_E4M3) *reinterpret_cast<uint32_t*>(r.a + u * 2048u + byte) = v[i];
+      if (r.mirror) *reinterpret_cast<uint32_t*>(r.mirror + u * r.mirror_unit + byte) = v[i];
+    }
+    w += 2;
+    w -= w >= n_bins ? n_bins : 0;
+  }
+}
+
+// Features [kb, ke) (multiples of 8) of one row.
+template <int PREC>
+HM_D void enc_units(const MlpDims& d, const float* __restrict__ xin, const float* __restrict__ enc_params, int kb,
+                    int ke, const EncRow& r) {
+  int done = kb;  // features before it are stored
+  for (int si = 0; si < d.n_segs; ++si) {
+    const EncSeg& s = d.segs[si];
+    if (s.type == ENC_IDENTITY) break;  // the last segment, with the padding below
+    const int lo = max(kb, s.out_off), hi = min(ke, s.out_off + s.n_out);
+    if (lo >= hi) continue;
+    done = hi;
+    const float* x = xin + s.in_off;
+    if (s.type == ENC_FREQUENCY) {
+      const int u = (lo - s.out_off) >> 1;
+      int dim = u / s.n_freq, f = u - dim * s.n_freq;
+      float xs = x[dim], p2 = scale_pow2(1.f, f);
+      for (int k = lo; k < hi; k += 8) {
+        float v[8];
+#pragma unroll
+        for (int t = 0; t < 4; ++t) {
+          sincospif(xs * p2, &v[2 * t], &v[2 * t + 1]);
+          p2 += p2;
+          if (++f == s.n_freq) {
+            f = 0;
+            p2 = 1.f;
+            xs = x[min(++dim, s.n_dims - 1)];
+          }
+        }
+        enc_store8<PREC>(r, k, v);
+      }
+    } else if (s.type == ENC_ONEBLOB) {
+      const int nb_i = s.n_bins;
+      const float nb = (float)nb_i, inv_nb = 1.f / nb;
+      const bool pow2 = (nb_i & (nb_i - 1)) == 0;  // then e * inv_nb is e / nb exactly
+      auto edge = [&](int e) { return pow2 ? (float)e * inv_nb : (float)e / nb; };
+      if (nb_i == 4) {  // two inputs per unit, every bin evaluated
+        for (int k = lo; k < hi; k += 8) {
+          const int dim = (k - s.out_off) >> 2;
+          float v[8];
+#pragma unroll
+          for (int t = 0; t < 2; ++t) {
+            const float c0 = oneblob_cdf(0.f, x[dim + t], nb);
+            float left = c0;
+#pragma unroll
+            for (int b = 0; b < 4; ++b) {
+              const float right = b == 3 ? c0 + 1.f : oneblob_cdf((float)(b + 1) * 0.25f, x[dim + t], nb);
+              v[4 * t + b] = right - left;
+              left = right;
+            }
+          }
+          enc_store8<PREC>(r, k, v);
+        }
+        continue;
+      }
+      int dim = (lo - s.out_off) / nb_i;
+      for (int k0 = s.out_off + dim * nb_i; k0 < hi; k0 += nb_i, ++dim) {
+        const int klo = max(lo, k0), khi = min(hi, k0 + nb_i);
+        const float zero[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+        for (int k = klo; k < khi; k += 8) enc_store8<PREC>(r, k, zero);
+        const float xv = x[dim];
+        // bin of x on the period [0, 1) (x itself may lie outside it)
+        int b0 = (int)floorf(xv * nb);
+        b0 = pow2 ? b0 & (nb_i - 1) : (b0 % nb_i + nb_i) % nb_i;
+        int first = b0 - 2;
+        first += first < 0 ? nb_i : 0;
+        // five masses from six edges; the edge after the last bin is edge 0
+        // of the next period, one full mass on
+        float m[5], left = oneblob_cdf(edge(first), xv, nb);
+        int e = first;
+#pragma unroll
+        for (int t = 0; t < 5; ++t) {
+          e = e + 1 == nb_i ? 0 : e + 1;
+          const float c = oneblob_cdf(edge(e), xv, nb);
+          m[t] = (e == 0 ? c + 1.f : c) - left;
+          left = c;
+        }
+        enc_store_window<PREC>(r, k0, nb_i, first, m, klo, khi);
+      }
+    } else {  // hash grid, two features per entry, four levels per unit
+      const float2* table = reinterpret_cast<const float2*>(enc_params + s.param_off);
+      const float px = x[0], py = x[1], pz = x[2];
+      for (int k = lo; k < hi; k += 8) {
+        float v[8];
+#pragma unroll
+        for (int t = 0; t < 4; ++t) {
+          const int l = ((k - s.out_off) >> 1) + t;
+          const float sc = s.level_scale[l];
+          const float fx = fmaf(sc, px, 0.5f), fy = fmaf(sc, py, 0.5f), fz = fmaf(sc, pz, 0.5f);
+          const float gx = floorf(fx), gy = floorf(fy), gz = floorf(fz);
+          const float wx = fx - gx, wy = fy - gy, wz = fz - gz;
+          uint32_t e[8];
+          grid_entries(s, l, (uint32_t)(int)gx, (uint32_t)(int)gy, (uint32_t)(int)gz, e);
+          float2 tv[8];  // eight gathers in flight
+#pragma unroll
+          for (int c = 0; c < 8; ++c) tv[c] = __ldg(table + e[c]);
+          float a0 = 0.f, a1 = 0.f;
+#pragma unroll
+          for (int c = 0; c < 8; ++c) {
+            const float w = ((c & 1) ? wx : 1.f - wx) * (((c >> 1) & 1) ? wy : 1.f - wy) *
+                            (((c >> 2) & 1) ? wz : 1.f - wz);
+            a0 += w * tv[c].x;
+            a1 += w * tv[c].y;
+          }
+          v[2 * t] = a0;
+          v[2 * t + 1] = a1;
+        }
+        enc_store8<PREC>(r, k, v);
+      }
+    }
+  }
+  // identity inputs, then padding: 1 up to in_pad, 0 past it
+  const EncSeg& s = d.segs[d.n_segs - 1];
+  for (int k = done; k < ke; k += 8) {
+    float v[8];
+#pragma unroll
+    for (int t = 0; t < 8; ++t) {
+      const int f = k + t;
+      v[t] = f < d.n_enc ? xin[s.in_off + f - s.out_off] : (f < d.in_pad ? 1.f : 0.f);
+    }
+    enc_store8<PREC>(r, k, v);
+  }
 }
 
 // Upper bound of |feature| over the row (E4M3 input scale).
@@ -469,6 +696,7 @@ struct TcArgs {
   // warp-specialised inference: shared-memory bytes of the weights, of one
   // layer-0 operand stage and of one hidden operand; number of stages
   int fz_w, fz_a0, fz_h, fz_stages;
+  int units;  // enc_units_ok and the hash tables 8-byte aligned
 };
 
 // Encoding of every row into the layer-0 operand, in the MMA's shared-memory
@@ -491,8 +719,13 @@ __global__ void __launch_bounds__(kTcRows) tc_encode_kernel(const __grid_constan
     row_scale = kE4M3Max / bound;
     if (valid) row_inv_out[q] = bound / kE4M3Max;
   }
-  RowPacker<PREC> pk(a_out + tile * p.tile_bytes, row, 0, row_scale);
   const int K0 = p.K[0];
+  if (valid && p.units) {
+    enc_units<PREC>(d, xin, p.enc_params, 0, K0,
+                    EncRow{a_out + tile * p.tile_bytes + op_offset(kTcRows, row, 0), nullptr, 0, row_scale});
+    return;
+  }
+  RowPacker<PREC> pk(a_out + tile * p.tile_bytes, row, 0, row_scale);
   if (valid) {
     enc_range<PREC>(d, xin, p.enc_params, 0, K0, pk);
   } else {
@@ -615,7 +848,11 @@ __global__ void __launch_bounds__(kTcThreads, 2) mlp_tc_fwd_kernel(const __grid_
           else
             pk.mirror = reinterpret_cast<uint8_t*>(p.x16 + q * K0 + kc);
         }
-        if (valid) {
+        if (valid && p.units) {
+          EncRow r{A + op_offset(kTcRows, row, 0) - (size_t)(kc / CK) * 2048, nullptr, 16, row_scale};
+          if (STORE) r.mirror = reinterpret_cast<uint8_t*>(p.x16 + q * K0);
+          enc_units<PREC>(d, xin, p.enc_params, kc + g0 * CK, kc + g1 * CK, r);
+        } else if (valid) {
           enc_range<PREC>(d, xin, p.enc_params, kc + g0 * CK, kc + g1 * CK, pk);
         } else {
           for (int k = g0 * CK; k < g1 * CK; ++k) pk.push(0.f);
@@ -793,11 +1030,12 @@ __global__ void __launch_bounds__(kFzThreads, 1) mlp_tc_fused_kernel(const __gri
       tc_fence_after();
       const uint32_t idesc = tc_idesc(kTcRows, p.N[l], FMT);
       const uint32_t b_lbo = 16 * p.N[l];
-      const uint32_t b_base = w_base + (uint32_t)p.boff[l];
+      uint64_t ad = tc_sdesc(a_base, a_lbo, 128);
+      uint64_t bd = tc_sdesc(w_base + (uint32_t)p.boff[l], b_lbo, 128);
       for (int ks = 0; ks < k_count / 16; ++ks) {
-        const uint64_t ad = tc_sdesc(a_base + (uint32_t)ks * 2 * a_lbo, a_lbo, 128);
-        const uint64_t bd = tc_sdesc(b_base + (uint32_t)ks * 2 * b_lbo, b_lbo, 128);
         tc_mma<false>(tm, ad, bd, idesc, ks > 0 ? 1u : 0u);
+        ad += 2 * a_lbo >> 4;  // the descriptors' start addresses, in 16-byte units
+        bd += 2 * b_lbo >> 4;
       }
       tc_commit(mma_s);
     };
@@ -805,20 +1043,18 @@ __global__ void __launch_bounds__(kFzThreads, 1) mlp_tc_fused_kernel(const __gri
       const int64_t tile = blockIdx.x + k * (int64_t)gridDim.x;
       if (tile >= n_tiles) break;
       const int st = (int)(k % NS);
+      // every thread waits for the MMAs itself (a leader polling for the group
+      // costs one more barrier per layer: 300 against 120 cycles).  A thread
+      // whose wait expired goes on to the group's barriers without waiting
+      // again, a leader without issuing, and the group stops at the tile's end.
       bool ok = true;
       if (leader) {
         ok = mbar_wait_bounded(full + st, (uint32_t)((k / NS) & 1));
-        if (ok) {
-          issue(0, smem_u32(A0 + st * p.fz_a0), K0);
-          ok = mbar_wait_bounded(mma_s, ph_mma);
-          if (ok) mbar_arrive(empty + st);  // the stage has been read
-        }
+        if (ok) issue(0, smem_u32(A0 + st * p.fz_a0), K0);
       }
+      ok = ok && mbar_wait_bounded(mma_s, ph_mma);
+      if (leader && ok) mbar_arrive(empty + st);  // the stage has been read
       ph_mma ^= 1u;
-      if (group_sync_or(bar_id, kFzLayWarps * 32, !ok)) {
-        failed = true;
-        break;
-      }
       tc_fence_after();
       for (int l = 1; l <= L; ++l) {
         // epilogue of layer l - 1: ReLU, rounded to the operand type, as the A of layer l
@@ -839,27 +1075,23 @@ __global__ void __launch_bounds__(kFzThreads, 1) mlp_tc_fused_kernel(const __gri
         tc_fence_before();
         fence_proxy_async_smem();
         group_sync(bar_id, kFzLayWarps * 32);
-        if (leader) {
-          issue(l, h_base, p.K[l]);
-          ok = mbar_wait_bounded(mma_s, ph_mma);
-        }
+        if (leader && ok) issue(l, h_base, p.K[l]);
+        ok = ok && mbar_wait_bounded(mma_s, ph_mma);
         ph_mma ^= 1u;
-        if (group_sync_or(bar_id, kFzLayWarps * 32, !ok)) {
-          failed = true;
-          break;
-        }
         tc_fence_after();
       }
-      if (failed) break;
       // output layer accumulator -> out
       float t[16];
       tmem_ld16(row_taddr, t);
       const int64_t q = tile * kTcRows + row;
-      if (q < p.n)
+      if (q < p.n && ok)
         for (int o = 0; o < d.out_ch && o < p.out_stride; ++o) p.out[q * p.out_stride + o] = t[o];
       // the next tile's layer-0 MMAs overwrite these columns
       tc_fence_before();
-      group_sync(bar_id, kFzLayWarps * 32);
+      if (group_sync_or(bar_id, kFzLayWarps * 32, !ok)) {
+        failed = true;
+        break;
+      }
     }
   } else {
     // ---------------- encoder team t (4 * P warps)
@@ -885,7 +1117,10 @@ __global__ void __launch_bounds__(kFzThreads, 1) mlp_tc_fused_kernel(const __gri
       }
       const int64_t q = tile * kTcRows + row;
       RowPacker<PREC> pk(As, row, g0, 1.f);
-      if (q < p.n) {
+      if (q < p.n && p.units) {
+        enc_units<PREC>(d, p.in + q * d.in_ch, p.enc_params, g0 * CK, g1 * CK,
+                        EncRow{As + op_offset(kTcRows, row, 0), nullptr, 0, 1.f});
+      } else if (q < p.n) {
         enc_range<PREC>(d, p.in + q * d.in_ch, p.enc_params, g0 * CK, g1 * CK, pk);
       } else {
         for (int kk = g0 * CK; kk < g1 * CK; ++kk) pk.push(0.f);
@@ -1110,6 +1345,9 @@ static int tc_args(const MlpDims& d, const TcPack& pk, const float* enc_params, 
     a.K[l] = l < pk.n_layers ? pk.K[l] : 0;
   }
   a.n_layers = pk.n_layers;
+  a.units = enc_units_ok(d) && (reinterpret_cast<uintptr_t>(enc_params) & 7) == 0;
+  for (int si = 0; si < d.n_segs; ++si)
+    if (d.segs[si].type == ENC_HASHGRID && d.segs[si].param_off % 2 != 0) a.units = 0;
   a.scales = pk.scales;
   a.enc_params = enc_params;
   a.in = in;
@@ -1152,12 +1390,6 @@ int64_t tc_encode_bytes(const MlpDims& d, const TcPack& pk, int64_t n) {
 // fit).  Set by hm_debug_tc_path.
 static int g_tc_path = 0;
 
-static bool has_hash_grid(const MlpDims& d) {
-  for (int si = 0; si < d.n_segs; ++si)
-    if (d.segs[si].type == ENC_HASHGRID) return true;
-  return false;
-}
-
 // Shared memory of mlp_tc_fused_kernel (0: the network does not fit it).
 static int64_t tc_fused_smem(const MlpDims& d, const TcPack& pk, TcArgs* a) {
   if (pk.precision == HM_PREC_FP8_E4M3 || (d.width != 32 && d.width != 64) || pk.N[pk.n_layers - 1] > d.width)
@@ -1198,8 +1430,7 @@ static int tc_fused_launch(const TcArgs& a, size_t smem, cudaStream_t st) {
 }
 
 bool tc_wants_workspace(const MlpDims& d, const TcPack& pk) {
-  if (g_tc_path == 2) return false;
-  return g_tc_path == 1 || has_hash_grid(d) || tc_fused_smem(d, pk, nullptr) == 0;
+  return g_tc_path != 2 && (g_tc_path == 1 || tc_fused_smem(d, pk, nullptr) == 0);
 }
 
 int tc_forward(const MlpDims& d, const TcPack& pk, const float* enc_params, const float* in, float* out,
@@ -1209,15 +1440,13 @@ int tc_forward(const MlpDims& d, const TcPack& pk, const float* enc_params, cons
   size_t smem = 0;
   if (int e = tc_args(d, pk, enc_params, in, out, out_stride, n, err_flag, &a, &smem)) return e;
   const bool have_work = work && work_bytes >= tc_encode_bytes(d, pk, n);
-  // Automatic choice, from the measured times (2^18 and 2^20 queries, W 64):
-  // with a workspace, the encode kernel + layer kernel where the encoding
-  // holds a hash grid (its table gathers are latency-bound and want the
-  // encode kernel's occupancy: 0.127 / 0.437 ms against 0.136 / 0.510), else
-  // the warp-specialised kernel (Frequency / OneBlob: 0.134 / 0.494 ms
-  // against 0.151 / 0.515); without one, the warp-specialised kernel
-  // wherever it fits (the layer kernel encoding its own tiles: 0.17 /
-  // 0.64 ms on either network).
-  const bool want_fz = g_tc_path == 2 || (g_tc_path == 0 && (!have_work || !has_hash_grid(d)));
+  // The warp-specialised kernel wherever it fits, from the measured times
+  // (FP16, width 64; 517 / 65,536 / 2^20 queries): 17 / 26 / 247 us on the
+  // Frequency / OneBlob network and 17 / 35 / 340 us on the hash grid, against
+  // 23 / 33 / 305 and 17 / 36 / 401 us for the encode kernel + layer kernel
+  // and 17 / 30 / 333 and 17 / 60 / 662 us for the layer kernel encoding its
+  // own tiles.
+  const bool want_fz = g_tc_path != 1;
   if (want_fz) {
     const int64_t fz = tc_fused_smem(d, pk, &a);
     if (fz > 0) {
