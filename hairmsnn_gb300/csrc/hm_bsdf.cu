@@ -19,13 +19,11 @@ HairConsts hair_consts_from_params(const hm_hair_params& p) { return hair_consts
 
 HM_D float ldg(const float* p) { return __ldg(p); }
 
-// Six 256-thread blocks per SM (40 registers; the eval needs 79 without
-// spilling, and spills about 250 bytes to L1 at 40): the kernels wait on the
-// latency of their transcendentals and dependent chains (a third of the
-// issue slots used at three blocks per SM), so more warps beat the spills.
-// Measured at 2^24 queries: eval 1.16 / 1.06 / 1.06 / 1.03 / 1.06 ms and
-// sample 1.59 / 1.47 / 1.50 / 1.45 / 1.46 ms at 3 / 4 / 5 / 6 / 8 blocks per
-// SM, results bit for bit the same.
+// Bound by instruction issue (about 1,500 and 1,900 instructions per query;
+// 75% of the issue slots used, 14% of HBM).  Six 256-thread blocks per SM (40
+// registers, a few spills to L1).  8,000,003 queries: eval 366 us, sample 463
+// at six blocks, 369 / 456 at four (before the lobe loop, the exact constant
+// divisions and the geometry shared by sample and evaluation: 493 / 700 us).
 __global__ void __launch_bounds__(256, 6) bsdf_eval_kernel(HairConsts hc, const float* __restrict__ wo,
                                                         const float* __restrict__ wi,
                                                         const float* __restrict__ t,

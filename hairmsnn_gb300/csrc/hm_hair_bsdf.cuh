@@ -71,6 +71,23 @@ HM_HD HairConsts hair_consts(const hm_hair_params& p) {
 // Host-side precompute of hair_consts (see hm_bsdf.cu).
 HairConsts hair_consts_from_params(const hm_hair_params& p);
 
+// a / c for a positive constant c whose reciprocal is a compile-time constant:
+// the quotient estimate, its exact remainder and one correction (Markstein,
+// IBM J. Res. Dev. 34, 1990), three instructions instead of a division's ten.
+// For every c used here this is the correctly rounded quotient of every
+// normal a (checked over all mantissas, tests/test_div_const.py), so results
+// keep their bits; a must not be infinite.
+HM_HD float div_const(float a, float c) {
+  const float y = 1.f / c;
+#ifdef __CUDA_ARCH__
+  const float q = __fmul_rn(a, y);
+  return __fmaf_rn(__fmaf_rn(-c, q, a), y, q);
+#else
+  const float q = a * y;
+  return fmaf(fmaf(-c, q, a), y, q);
+#endif
+}
+
 HM_D float bessel_i0(float x) {  // disney_hair.cuh:54-67
   float val = 0.f, x2i = 1.f;
   float ifact = 1.f;  // i! for i <= 9 is exact in float (int64 in the reference)
@@ -78,16 +95,19 @@ HM_D float bessel_i0(float x) {  // disney_hair.cuh:54-67
 #pragma unroll
   for (int i = 0; i < 10; ++i) {
     if (i > 1) ifact *= (float)i;
-    val += x2i / (i4 * sqr(ifact));
+    val += div_const(x2i, i4 * sqr(ifact));
     x2i *= x * x;
     i4 *= 4.f;
   }
   return val;
 }
 
-HM_D float log_i0(float x) {  // disney_hair.cuh:70-75; the `0.5 *` product is FP64
-  if (x > 12.f)
-    return (float)((double)x + 0.5 * (double)(-logf(2.f * kPi) + logf(1.f / x) + 1.f / (8.f * x)));
+// disney_hair.cuh:70-75.  The reference forms x + 0.5 * g in FP64 and rounds
+// to float; that FP64 sum is exact (x in (12, 1 / v], v > 0.0015 where this
+// branch runs, and |g| > 4 span at most 50 bits), so one fused multiply-add
+// gives the same float without the FP64 units.
+HM_D float log_i0(float x) {
+  if (x > 12.f) return __fmaf_rn(0.5f, -logf(2.f * kPi) + logf(1.f / x) + 1.f / (8.f * x), x);
   return logf(bessel_i0(x));
 }
 
@@ -103,17 +123,24 @@ HM_D double bessel_i0_d(double x) {
   return val;
 }
 
+// The log-space branch of M_p in FP64.  One copy of the code, called: inlined
+// into every lobe of every evaluation its logarithms and exponential made the
+// kernels larger than the instruction caches: five to eight issue slots lost
+// to fetching for each instruction of the shading kernel, and bsdf_eval_kernel
+// took 36 us for 262,144 queries instead of 22.
+static __device__ __noinline__ float mp_lobe_fp64(float cti, float cto, float sti, float sto, float v) {
+  double dv = v;
+  double a = (double)cti * (double)cto / dv;
+  double b = (double)sti * (double)sto / dv;
+  double li = a > 12.0 ? a + 0.5 * (-log(2.0 * (double)kPi) + log(1.0 / a) + 1.0 / (8.0 * a))
+                       : log(bessel_i0_d(a));
+  return (float)exp(li - b - 1.0 / dv + 0.6931 + log(1.0 / (2.0 * dv)));
+}
+
 // M_p (disney_hair.cuh:78-88) for lobe constants k; v = v[k].
 HM_D float mp_lobe(float cti, float cto, float sti, float sto, const HairConsts& hc, int k) {
   const float v = hc.v[k];
-  if (hc.fp64_mp && v <= 0.1f) {
-    double dv = v;
-    double a = (double)cti * (double)cto / dv;
-    double b = (double)sti * (double)sto / dv;
-    double li = a > 12.0 ? a + 0.5 * (-log(2.0 * (double)kPi) + log(1.0 / a) + 1.0 / (8.0 * a))
-                         : log(bessel_i0_d(a));
-    return (float)exp(li - b - 1.0 / dv + 0.6931 + log(1.0 / (2.0 * dv)));
-  }
+  if (hc.fp64_mp && v <= 0.1f) return mp_lobe_fp64(cti, cto, sti, sto, v);
   float a = cti * cto / v;
   float b = sti * sto / v;
   if (v <= 0.1f) return expf(log_i0(a) - b - hc.inv_v[k] + 0.6931f + hc.mp_logc[k]);
@@ -139,112 +166,109 @@ struct HairEval {
   float pdf;  // full 4-lobe mixture pdf
 };
 
-// disney_hair(si, &pdf), disney_hair.cuh:186-266.  wo, wi: hair-frame unit
-// vectors (x along the fibre); h = dot(Y, n) in [-1, 1].
-HM_D HairEval hair_eval(f3 wo, f3 wi, float h, const HairConsts& hc) {
+// What an evaluation or a sample needs of (wo, h, material) alone: computed
+// once for a vertex and shared by its light sample, BSDF sample and next
+// direction (each once computed it again).
+struct HairGeom {
+  float sin_to, cos_to, phi_o, gamma_o, gamma_t;
+  float fr;       // Fresnel, the R lobe's attenuation
+  f3 a1, a2, a3;  // TT, TRT, TRRT attenuations
+  float ap[4];    // lobe pmf
+};
+
+// disney_hair.cuh:186-218 and computeApPdf (:143-182; with eta = Eta it reuses
+// the T and Fresnel of the evaluation).  wo: hair-frame unit vector (x along
+// the fibre); h = dot(Y, n) in [-1, 1].
+HM_D HairGeom hair_geom(f3 wo, float h, const HairConsts& hc) {
+  HairGeom g;
   const float sin_to = wo.x;
   const float cos_to = safe_sqrt(1.f - sqr(sin_to));
-  const float phi_o = atan2f(wo.z, wo.y);
-  const float sin_ti = wi.x;
-  const float cos_ti = safe_sqrt(1.f - sqr(sin_ti));
-  const float phi_i = atan2f(wi.z, wi.y);
-  const float sin_tt = sin_to / kEta;
+  g.sin_to = sin_to;
+  g.cos_to = cos_to;
+  g.phi_o = atan2f(wo.z, wo.y);
+  const float sin_tt = div_const(sin_to, kEta);
   const float cos_tt = safe_sqrt(1.f - sqr(sin_tt));
-  const float gamma_o = asinf(h);
-  const float cos_go = cosf(gamma_o);
+  g.gamma_o = asinf(h);
+  const float cos_go = cosf(g.gamma_o);
   const float etap = sqrtf(kEta * kEta - sqr(sin_to)) / cos_to;
   const float sin_gt = h / etap;
   const float cos_gt = safe_sqrt(1.f - sqr(sin_gt));
-  const float gamma_t = safe_asin(sin_gt);
+  g.gamma_t = safe_asin(sin_gt);
   const float fac = (2.f * cos_gt / cos_tt);
   const f3 T = mk(expf(-hc.sigma_a[0] * fac), expf(-hc.sigma_a[1] * fac), expf(-hc.sigma_a[2] * fac));
   // Fresnel(Eta, cos_to * cos_go), disney_hair.cuh:46-51
   const float F0 = sqr(1.f - kEta) / sqr(1.f + kEta);
   const float xd = 1.f - cos_to * cos_go;
   const float fr = F0 + (1.f - F0) * xd * xd * xd * xd * xd;
+  g.fr = fr;
   // A_p, :91-109
-  const f3 a0 = splat(fr);
-  const f3 a1 = sqr(1.f - fr) * T;
-  const f3 a2 = sqr(1.f - fr) * T * T * fr;
-  const f3 a3 = a2 * fr * T / (splat(1.f) - T * fr);
-  const float phi = phi_i - phi_o;
-
-  float sop = sin_to * hc.cos2k[1] - cos_to * hc.sin2k[1];
-  float cop = fabsf(cos_to * hc.cos2k[1] + sin_to * hc.sin2k[1]);
-  const float mp0 = mp_lobe(cos_ti, cop, sin_ti, sop, hc, 0);
-  const float np0 = np_lobe(phi, 0, gamma_o, gamma_t, hc);
-  f3 f = hc.gain[0] * mp0 * a0 * np0;
-
-  sop = sin_to * hc.cos2k[0] + cos_to * hc.sin2k[0];
-  cop = fabsf(cos_to * hc.cos2k[0] - sin_to * hc.sin2k[0]);
-  const float mp1 = mp_lobe(cos_ti, cop, sin_ti, sop, hc, 1);
-  const float np1 = np_lobe(phi, 1, gamma_o, gamma_t, hc);
-  f = f + hc.gain[1] * mp1 * a1 * np1;
-
-  sop = sin_to * hc.cos2k[2] + cos_to * hc.sin2k[2];
-  cop = fabsf(cos_to * hc.cos2k[2] - sin_to * hc.sin2k[2]);
-  const float mp2 = mp_lobe(cos_ti, cop, sin_ti, sop, hc, 2);
-  const float np2 = np_lobe(phi, 2, gamma_o, gamma_t, hc);
-  f = f + hc.gain[2] * mp2 * a2 * np2;
-
-  const float mpm = mp_lobe(cos_ti, cos_to, sin_ti, sin_to, hc, 2);
-  const float npm = 1.f / (2.f * kPi);
-  f = f + hc.gain[3] * mpm * a3 * npm;
-
-  // computeApPdf (:143-182): with eta = Eta it reuses the T and Fresnel above.
-  float ap[4] = {(a0.x + a0.y + a0.z) / 3.f, (a1.x + a1.y + a1.z) / 3.f,
-                 (a2.x + a2.y + a2.z) / 3.f, (a3.x + a3.y + a3.z) / 3.f};
+  g.a1 = sqr(1.f - fr) * T;
+  g.a2 = sqr(1.f - fr) * T * T * fr;
+  g.a3 = g.a2 * fr * T / (splat(1.f) - T * fr);
+  const float ap[4] = {(fr + fr + fr) / 3.f, (g.a1.x + g.a1.y + g.a1.z) / 3.f, (g.a2.x + g.a2.y + g.a2.z) / 3.f,
+                       (g.a3.x + g.a3.y + g.a3.z) / 3.f};
   const float sum = ap[0] + ap[1] + ap[2] + ap[3];
+#pragma unroll
+  for (int p = 0; p < 4; ++p) g.ap[p] = ap[p] / sum;
+  return g;
+}
+
+// disney_hair(si, &pdf), disney_hair.cuh:186-266, for the geometry of (wo, h).
+// wi: hair-frame unit vector.
+HM_D HairEval hair_eval(const HairGeom& g, f3 wi, const HairConsts& hc) {
+  const float sin_to = g.sin_to, cos_to = g.cos_to;
+  const float sin_ti = wi.x;
+  const float cos_ti = safe_sqrt(1.f - sqr(sin_ti));
+  const float phi_i = atan2f(wi.z, wi.y);
+  const float phi = phi_i - g.phi_o;
+
+  // M_p and N_p of the lobes R, TT, TRT, TRRT.  R tilts by -2^1 alpha, TT by
+  // 2^0, TRT by 2^2, TRRT not (the sine's sign carries the direction exactly).
+  // A loop, not unrolled: the four copies of a lobe's code overran the
+  // instruction caches.  bsdf_sample_kernel, 8,000,003 queries: 672 us
+  // unrolled, 632 as a loop; its sums f and pdf stay outside the loop (713
+  // inside it, with the values they keep alive).
+  float mp[4], np[3];
+#pragma unroll 1
+  for (int p = 0; p < 4; ++p) {
+    float sop = sin_to, cop = cos_to;
+    if (p < 3) {
+      const int k = p == 0 ? 1 : (p == 1 ? 0 : 2);
+      const float sk = p == 0 ? -hc.sin2k[k] : hc.sin2k[k], ck = hc.cos2k[k];
+      sop = sin_to * ck + cos_to * sk;
+      cop = fabsf(cos_to * ck - sin_to * sk);
+      np[p] = np_lobe(phi, p, g.gamma_o, g.gamma_t, hc);
+    }
+    mp[p] = mp_lobe(cos_ti, cop, sin_ti, sop, hc, p < 3 ? p : 2);
+  }
+  const float npm = 1.f / (2.f * kPi);
+  f3 f = hc.gain[0] * mp[0] * splat(g.fr) * np[0];
+  f = f + hc.gain[1] * mp[1] * g.a1 * np[1];
+  f = f + hc.gain[2] * mp[2] * g.a2 * np[2];
+  f = f + hc.gain[3] * mp[3] * g.a3 * npm;
   float pdf = 0.f;
-  pdf = pdf + mp0 * (ap[0] / sum) * np0;
-  pdf = pdf + mp1 * (ap[1] / sum) * np1;
-  pdf = pdf + mp2 * (ap[2] / sum) * np2;
-  pdf = pdf + mpm * (ap[3] / sum) * npm;
+  pdf = pdf + mp[0] * g.ap[0] * np[0];
+  pdf = pdf + mp[1] * g.ap[1] * np[1];
+  pdf = pdf + mp[2] * g.ap[2] * np[2];
+  pdf = pdf + mp[3] * g.ap[3] * npm;
   return HairEval{f, pdf};
 }
 
-// Lobe-selection pmf (computeApPdf, disney_hair.cuh:143-182).
-HM_D void hair_ap_pdf(float sin_to, float cos_to, float cos_go, float h, const HairConsts& hc,
-                      float out[4]) {
-  const float sin_tt = sin_to / kEta;
-  const float cos_tt = safe_sqrt(1.f - sqr(sin_tt));
-  const float etap = sqrtf(kEta * kEta - sqr(sin_to)) / cos_to;
-  const float sin_gt = h / etap;
-  const float cos_gt = safe_sqrt(1.f - sqr(sin_gt));
-  const float fac = (2.f * cos_gt / cos_tt);
-  const f3 T = mk(expf(-hc.sigma_a[0] * fac), expf(-hc.sigma_a[1] * fac), expf(-hc.sigma_a[2] * fac));
-  const float F0 = sqr(1.f - kEta) / sqr(1.f + kEta);
-  const float xd = 1.f - cos_to * cos_go;
-  const float fr = F0 + (1.f - F0) * xd * xd * xd * xd * xd;
-  const f3 a1 = sqr(1.f - fr) * T;
-  const f3 a2 = sqr(1.f - fr) * T * T * fr;
-  const f3 a3 = a2 * fr * T / (splat(1.f) - T * fr);
-  out[0] = (fr + fr + fr) / 3.f;
-  out[1] = (a1.x + a1.y + a1.z) / 3.f;
-  out[2] = (a2.x + a2.y + a2.z) / 3.f;
-  out[3] = (a3.x + a3.y + a3.z) / 3.f;
-  const float sum = out[0] + out[1] + out[2] + out[3];
-#pragma unroll
-  for (int p = 0; p < 4; ++p) out[p] = out[p] / sum;
-}
+HM_D HairEval hair_eval(f3 wo, f3 wi, float h, const HairConsts& hc) { return hair_eval(hair_geom(wo, h, hc), wi, hc); }
 
-// sample_disney_hair(si, rand, &pdf), disney_hair.cuh:277-386.  Returns the
-// hair-frame wi and the full eval at it.  The TRRT lobe (p = 3) uses
-// v[3] == s: in the reference's HairInteraction the element after v[2] is s.
-HM_D HairEval hair_sample(f3 wo, float h, float u0, float u1, float u2, float u3,
-                          const HairConsts& hc, f3* wi_out) {
-  const float sin_to = wo.x;
-  const float cos_to = safe_sqrt(1.f - sqr(sin_to));
-  const float phi_o = atan2f(wo.z, wo.y);
-  const float gamma_o = asinf(h);
-  const float cos_go = cosf(gamma_o);
-  float ap[4];
-  hair_ap_pdf(sin_to, cos_to, cos_go, h, hc, ap);
+// The direction of sample_disney_hair (hair frame).  The TRRT lobe (p = 3)
+// uses v[3] == s: in the reference's HairInteraction the element after v[2]
+// is s.
+HM_D f3 hair_sample_dir(const HairGeom& g, float u0, float u1, float u2, float u3, const HairConsts& hc) {
+  const float sin_to = g.sin_to, cos_to = g.cos_to;
   int p = 0;
   float eps1 = u0;
-  for (p = 0; p < 3; ++p) {
-    if (eps1 < ap[p]) break;
-    eps1 -= ap[p];
+#pragma unroll
+  for (int k = 0; k < 3; ++k) {
+    if (p == k && !(eps1 < g.ap[k])) {
+      eps1 -= g.ap[k];
+      p = k + 1;
+    }
   }
   float sop, cop;
   if (p == 0) {
@@ -267,20 +291,25 @@ HM_D HairEval hair_sample(f3 wo, float h, float u0, float u1, float u2, float u3
   const float cos_phi = cosf(2.f * kPi * u2);
   const float sin_ti = -cos_theta * sop + sin_theta * cos_phi * cop;
   const float cos_ti = safe_sqrt(1.f - sqr(sin_ti));
-  const float etap = sqrtf(kEta * kEta - sqr(sin_to)) / cos_to;
-  const float gamma_t = safe_asin(h / etap);
   float dphi;
   if (p < 3) {
     // SampleTrimmedLogistic(u3, s, -pi, pi), :269-274
     float x = -hc.s * logf(1.f / (u3 * hc.trim_den + hc.cdf_lo) - 1.f);
-    dphi = phi_p(p, gamma_o, gamma_t) + fminf(fmaxf(x, -kPi), kPi);
+    dphi = phi_p(p, g.gamma_o, g.gamma_t) + fminf(fmaxf(x, -kPi), kPi);
   } else {
     dphi = 2.f * kPi * u3;
   }
-  const float phi_i = phi_o + dphi;
-  const f3 wi = normalize(mk(sin_ti, cos_ti * cosf(phi_i), cos_ti * sinf(phi_i)));
-  *wi_out = wi;
-  return hair_eval(wo, wi, h, hc);
+  const float phi_i = g.phi_o + dphi;
+  return normalize(mk(sin_ti, cos_ti * cosf(phi_i), cos_ti * sinf(phi_i)));
+}
+
+// sample_disney_hair(si, rand, &pdf), disney_hair.cuh:277-386.  Returns the
+// hair-frame wi and the full eval at it.
+HM_D HairEval hair_sample(f3 wo, float h, float u0, float u1, float u2, float u3,
+                          const HairConsts& hc, f3* wi_out) {
+  const HairGeom g = hair_geom(wo, h, hc);
+  *wi_out = hair_sample_dir(g, u0, u1, u2, u3, hc);
+  return hair_eval(g, *wi_out, hc);
 }
 
 // Hair shading frame of the reference's closest-hit program

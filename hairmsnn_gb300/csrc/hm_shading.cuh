@@ -251,6 +251,18 @@ HM_D f3 curve_surface_normal(const Cubic& bc, float u, f3* ps) {
 }
 
 // ------------------------------------------------------------ vertex (closest hit)
+// One copy of the BSDF's code each, called (see mp_lobe_fp64).
+static __device__ __noinline__ void hair_geom_call(f3 wo, float h, const HairConsts* hc, HairGeom* g) {
+  *g = hair_geom(wo, h, *hc);
+}
+static __device__ __noinline__ HairEval hair_eval_call(const HairGeom* g, f3 wi, const HairConsts* hc) {
+  return hair_eval(*g, wi, *hc);
+}
+static __device__ __noinline__ f3 hair_sample_call(const HairGeom* g, float u0, float u1, float u2, float u3,
+                                                   const HairConsts* hc) {
+  return hair_sample_dir(*g, u0, u1, u2, u3, *hc);
+}
+
 struct Vertex {
   f3 p, n, t, wo;
   Frame fr;
@@ -260,6 +272,7 @@ struct Vertex {
   int group;                  // strand group (0 for the surface)
   const HairConsts* hc;       // material that samples and weighs (pdfs, MIS)
   const HairConsts* hc_eval;  // material of the BSDF values (== hc but in detached renders)
+  HairGeom geom;              // hair: what hc's BSDF needs of wo_local and h
 };
 
 // The traversal's hit recomputed for its own primitive with every operation
@@ -329,7 +342,15 @@ HM_D Vertex setup_vertex(const SceneDev& s, f3 ro, f3 rd, const float4 hit) {
   }
   v.hc_eval = v.hc;
   v.wo_local = normalize(to_local(v.fr, v.wo));
+  if (!v.surface) hair_geom_call(v.wo_local, dot(v.fr.r1, v.n), v.hc, &v.geom);
   return v;
+}
+
+// The BSDF value of the evaluation material (detached renders).
+HM_D f3 hair_f_detached(const Vertex& v, f3 wi_local) {
+  HairGeom g;
+  hair_geom_call(v.wo_local, dot(v.fr.r1, v.n), v.hc_eval, &g);
+  return hair_eval_call(&g, wi_local, v.hc_eval).f;
 }
 
 // One light-transport sample whose value counts only if its shadow ray is unoccluded.
@@ -344,9 +365,9 @@ HM_D f3 bsdf_eval_vertex(const SceneDev& s, const Vertex& v, f3 wi_local, float*
   if (!v.surface) {
     f3 n_local = v.n;  // unused by the eval; h is taken from the frame
     (void)n_local;
-    HairEval e = hair_eval(v.wo_local, wi_local, dot(v.fr.r1, v.n), *v.hc);
+    HairEval e = hair_eval_call(&v.geom, wi_local, v.hc);
     *pdf = e.pdf;
-    if (v.hc_eval != v.hc) return hair_eval(v.wo_local, wi_local, dot(v.fr.r1, v.n), *v.hc_eval).f;
+    if (v.hc_eval != v.hc) return hair_f_detached(v, wi_local);
     return e.f;
   }
   f3 f = frostbite_ggx(v.wo_local, wi_local, s.diffuse, s.alpha);
@@ -408,10 +429,11 @@ HM_D ShadowSample sample_bsdf(const SceneDev& s, const Vertex& v, f3* p, uint32_
   f3 bsdf, wi_local;
   if (!v.surface) {
     float r2 = lcg_next(rng), r3 = lcg_next(rng);
-    HairEval e = hair_sample(v.wo_local, dot(v.fr.r1, v.n), r0, r1, r2, r3, *v.hc, &wi_local);
+    wi_local = hair_sample_call(&v.geom, r0, r1, r2, r3, v.hc);
+    HairEval e = hair_eval_call(&v.geom, wi_local, v.hc);
     bsdf = e.f;
     bsdfPdf = e.pdf;
-    if (v.hc_eval != v.hc) bsdf = hair_eval(v.wo_local, wi_local, dot(v.fr.r1, v.n), *v.hc_eval).f;
+    if (v.hc_eval != v.hc) bsdf = hair_f_detached(v, wi_local);
   } else {
     wi_local = sample_ggx(r0, r1, s.alpha, v.wo_local, &bsdfPdf);
     bsdf = frostbite_ggx(v.wo_local, wi_local, s.diffuse, s.alpha);
@@ -461,11 +483,12 @@ HM_D f3 next_vertex(const SceneDev& s, const Vertex& v, uint32_t& rng, f3* ro, f
   f3 bsdf, wi_local, bsdf_s;
   if (!v.surface) {
     float r2 = lcg_next(rng), r3 = lcg_next(rng);
-    HairEval e = hair_sample(v.wo_local, dot(v.fr.r1, v.n), r0, r1, r2, r3, *v.hc, &wi_local);
+    wi_local = hair_sample_call(&v.geom, r0, r1, r2, r3, v.hc);
+    HairEval e = hair_eval_call(&v.geom, wi_local, v.hc);
     bsdf = e.f;
     pdf = e.pdf;
     bsdf_s = bsdf;
-    if (v.hc_eval != v.hc) bsdf = hair_eval(v.wo_local, wi_local, dot(v.fr.r1, v.n), *v.hc_eval).f;
+    if (v.hc_eval != v.hc) bsdf = hair_f_detached(v, wi_local);
   } else {
     wi_local = sample_ggx(r0, r1, s.alpha, v.wo_local, &pdf);
     bsdf = frostbite_ggx(v.wo_local, wi_local, s.diffuse, s.alpha);
