@@ -728,6 +728,11 @@ __global__ void adam_kernel(float* __restrict__ w, const float* __restrict__ g, 
   }
 }
 
+__global__ void unscale_kernel(const float* __restrict__ g, float inv, float* __restrict__ out, int64_t n) {
+  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
+    out[i] = g[i] * inv;
+}
+
 // ====================================================================== state
 struct Mlp {
   MlpConfig cfg;
@@ -735,6 +740,7 @@ struct Mlp {
   int64_t n_params = 0;
   float* params = nullptr;  // [net | enc]
   float* grads = nullptr;
+  float* grads_out = nullptr;  // gradients without the loss scale (hm_mlp_get_gradients)
   float* adam_m = nullptr;
   float* adam_v = nullptr;
   int step = 0;
@@ -982,6 +988,7 @@ extern "C" void hm_mlp_destroy(hm_mlp* h) {
   free_ws(m);
   cudaFree(m->params);
   cudaFree(m->grads);
+  cudaFree(m->grads_out);
   cudaFree(m->adam_m);
   cudaFree(m->adam_v);
   cudaFree(m->dw_part);
@@ -1029,11 +1036,21 @@ extern "C" int hm_mlp_set_params(hm_mlp* h, const float* host_in) {
 }
 
 extern "C" int hm_mlp_get_gradients(const hm_mlp* h, float* host_out) {
-  const Mlp* m = (const Mlp*)h;
+  Mlp* m = const_cast<Mlp*>((const Mlp*)h);  // grads_out is a lazily made buffer
   if (!m || !host_out) return hm_set_error("hm_mlp_get_gradients: NULL"), HM_EINVAL;
-  cudaError_t e = cudaMemcpy(host_out, m->grads, m->n_params * sizeof(float), cudaMemcpyDeviceToHost);
-  if (e == cudaSuccess && m->tc_train && m->loss_scale != 1.f)  // undo the FP16 loss scale
-    for (int64_t i = 0; i < m->n_params; ++i) host_out[i] /= m->loss_scale;
+  const float* src = m->grads;
+  cudaError_t e = cudaSuccess;
+  if (m->tc_train && m->loss_scale != 1.f) {
+    // undo the FP16 loss scale (a power of two: exact) on the device: over the
+    // renderer's million gradients the host loop took 0.2 ms of a 0.43 ms step
+    if (!m->grads_out) e = cudaMalloc(&m->grads_out, m->n_params * sizeof(float));
+    if (e == cudaSuccess) {
+      unscale_kernel<<<1024, 256>>>(m->grads, 1.f / m->loss_scale, m->grads_out, m->n_params);
+      e = cudaGetLastError();
+      src = m->grads_out;
+    }
+  }
+  if (e == cudaSuccess) e = cudaMemcpy(host_out, src, m->n_params * sizeof(float), cudaMemcpyDeviceToHost);
   return e == cudaSuccess ? HM_OK : hm_cuda_status(e, "hm_mlp_get_gradients");
 }
 

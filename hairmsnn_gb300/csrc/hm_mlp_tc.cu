@@ -1138,11 +1138,29 @@ __global__ void __launch_bounds__(kFzThreads, 1) mlp_tc_fused_kernel(const __gri
 }
 
 // ------------------------------------------------------------ weight packing
-__global__ void tc_scales_kernel(MlpDims d, const float* __restrict__ params, int n_layers, float* __restrict__ scales) {
-  // block l < n_layers: amax of layer l's weights -> 1 / (448 / amax);
-  // block n_layers: amax of the encoding parameters (hash tables)
-  __shared__ float red[256];
-  const int l = blockIdx.x;
+// All layers in one launch: blockIdx.y the layer, blockIdx.z 0 for the
+// forward operand, 1 for the transposed one of the backward pass (a launch
+// per layer and direction cost 36 us before every training step of the
+// 5 x 64 network, one costs 4).
+struct TcPackArgs {
+  MlpDims d;
+  const float* params;
+  int n_layers;
+  int N[16], K[16], NT[16], KT[16];
+  int64_t boff[16], boff_t[16];
+  uint8_t* blob;
+  uint8_t* blob_t;  // W_l^T: element (n = input, k = output) of layer l
+  float* scales;    // [16] weight scales (E4M3; [15]: hash-grid amax)
+  const uint32_t* amax;  // [16] largest |weight| as float bits, from tc_amax_kernel
+};
+
+// E4M3: amax of layer blockIdx.y's weights, blockIdx.y == n_layers: of the
+// encoding parameters (as integers: the bits of non-negative floats order as
+// the floats do, so the result does not depend on the blocks' order).
+__global__ void __launch_bounds__(256) tc_amax_kernel(const __grid_constant__ MlpDims d, const float* __restrict__ params,
+                                                      int n_layers, uint32_t* __restrict__ amax) {
+  __shared__ float red[8];
+  const int l = blockIdx.y;
   int64_t begin, count;
   if (l < n_layers) {
     const int fan_in = l == 0 ? d.in_pad : d.width;
@@ -1154,55 +1172,55 @@ __global__ void tc_scales_kernel(MlpDims d, const float* __restrict__ params, in
     count = d.n_enc_params;
   }
   float m = 0.f;
-  for (int64_t i = threadIdx.x; i < count; i += blockDim.x) m = fmaxf(m, fabsf(params[begin + i]));
-  red[threadIdx.x] = m;
+  for (int64_t i = blockIdx.x * 256 + threadIdx.x; i < count; i += (int64_t)gridDim.x * 256)
+    m = fmaxf(m, fabsf(params[begin + i]));
+  for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
+  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = m;
   __syncthreads();
-  for (int w = 128; w > 0; w >>= 1) {
-    if (threadIdx.x < w) red[threadIdx.x] = fmaxf(red[threadIdx.x], red[threadIdx.x + w]);
-    __syncthreads();
-  }
   if (threadIdx.x == 0) {
-    if (l < n_layers)
-      scales[l] = red[0] > 0.f ? red[0] / kE4M3Max : 1.f;
-    else
-      scales[15] = red[0];
+    for (int w = 1; w < 8; ++w) m = fmaxf(m, red[w]);
+    if (m > 0.f) atomicMax(amax + (l < n_layers ? l : 15), __float_as_uint(m));
   }
 }
 
 template <int PREC>
-__global__ void tc_pack_kernel(MlpDims d, const float* __restrict__ params, int layer, int N, int K,
-                               int64_t boff, const float* __restrict__ scales, uint8_t* __restrict__ blob) {
-  const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+__global__ void __launch_bounds__(256) tc_pack_kernel(const __grid_constant__ TcPackArgs p) {
+  const int l = blockIdx.y;
+  const int64_t i = blockIdx.x * 256 + threadIdx.x;
+  const int fan_in = l == 0 ? p.d.in_pad : p.d.width;
+  const float* W = p.params + p.d.layer_off[l];
+  if (blockIdx.z == 1) {  // transposed, FP16 / BF16
+    if (i >= (int64_t)p.NT[l] * p.KT[l]) return;
+    const int n = (int)(i / p.KT[l]), k = (int)(i % p.KT[l]);
+    const float w = n < fan_in ? W[(int64_t)k * fan_in + n] : 0.f;
+    uint8_t* dst = p.blob_t + p.boff_t[l] + op_offset(p.NT[l], n, 2 * k);
+    if (PREC == TC_BF16)
+      *reinterpret_cast<__nv_bfloat16*>(dst) = __float2bfloat16_rn(w);
+    else
+      *reinterpret_cast<__half*>(dst) = __float2half_rn(w);
+    return;
+  }
+  const int N = p.N[l], K = p.K[l];
+  float scale = 1.f;
+  if (PREC == TC_E4M3) {
+    const float m = __uint_as_float(p.amax[l]);
+    scale = m > 0.f ? m / kE4M3Max : 1.f;
+    if (i == 0) p.scales[l] = scale;
+    if (i == 0 && l == 0) p.scales[15] = __uint_as_float(p.amax[15]);
+  }
   if (i >= (int64_t)N * K) return;
   const int n = (int)(i / K), k = (int)(i % K);
-  const int fan_in = layer == 0 ? d.in_pad : d.width;
-  const float w = k < fan_in ? params[d.layer_off[layer] + (int64_t)n * fan_in + k] : 0.f;
+  const float w = k < fan_in ? W[(int64_t)n * fan_in + k] : 0.f;
+  uint8_t* blob = p.blob + p.boff[l];
   if (PREC == TC_E4M3) {
-    const float s = 1.f / scales[layer];
+    const float s = 1.f / scale;
     const uint32_t v = __nv_cvt_float2_to_fp8x2(make_float2(w * s, 0.f), __NV_SATFINITE, __NV_E4M3);
-    blob[boff + op_offset(N, n, k)] = (uint8_t)(v & 0xFF);
+    blob[op_offset(N, n, k)] = (uint8_t)(v & 0xFF);
   } else if (PREC == TC_BF16) {
-    __nv_bfloat16 h = __float2bfloat16_rn(w);
-    *reinterpret_cast<__nv_bfloat16*>(blob + boff + op_offset(N, n, 2 * k)) = h;
+    *reinterpret_cast<__nv_bfloat16*>(blob + op_offset(N, n, 2 * k)) = __float2bfloat16_rn(w);
   } else {
-    __half h = __float2half_rn(w);
-    *reinterpret_cast<__half*>(blob + boff + op_offset(N, n, 2 * k)) = h;
+    *reinterpret_cast<__half*>(blob + op_offset(N, n, 2 * k)) = __float2half_rn(w);
   }
-}
-
-// W_l^T for the backward pass: element (n = input, k = output) of layer l.
-template <int PREC>
-__global__ void tc_pack_t_kernel(MlpDims d, const float* __restrict__ params, int layer, int NT, int KT,
-                                 int64_t boff, uint8_t* __restrict__ blob) {
-  const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  if (i >= (int64_t)NT * KT) return;
-  const int n = (int)(i / KT), k = (int)(i % KT);
-  const int fan_in = layer == 0 ? d.in_pad : d.width;
-  const float w = n < fan_in ? params[d.layer_off[layer] + (int64_t)k * fan_in + n] : 0.f;
-  if (PREC == TC_BF16)
-    *reinterpret_cast<__nv_bfloat16*>(blob + boff + op_offset(NT, n, 2 * k)) = __float2bfloat16_rn(w);
-  else
-    *reinterpret_cast<__half*>(blob + boff + op_offset(NT, n, 2 * k)) = __float2half_rn(w);
 }
 
 // ------------------------------------------------------------------ host API
@@ -1254,7 +1272,7 @@ int tc_pack_alloc(const MlpDims& d, int precision, TcPack* pk) {
   }
   pk->bytes = off;
   cudaError_t e = cudaMalloc(&pk->blob, (size_t)off);
-  if (e == cudaSuccess) e = cudaMalloc(&pk->scales, 16 * sizeof(float));
+  if (e == cudaSuccess) e = cudaMalloc(&pk->scales, 32 * sizeof(float));  // [16..31]: amax bits
   if (e == cudaSuccess && tc_trainable(d, precision)) {
     int64_t ot = 0;
     for (int l = 0; l < pk->n_layers; ++l) {
@@ -1267,7 +1285,7 @@ int tc_pack_alloc(const MlpDims& d, int precision, TcPack* pk) {
     e = cudaMalloc(&pk->blob_t, (size_t)ot);
   }
   if (e != cudaSuccess) return hm_cuda_status(e, "tensor-core weight blob");
-  cudaMemset(pk->scales, 0, 16 * sizeof(float));
+  cudaMemset(pk->scales, 0, 32 * sizeof(float));
   return HM_OK;
 }
 
@@ -1281,30 +1299,42 @@ void tc_pack_free(TcPack* pk) {
 }
 
 int tc_pack(const MlpDims& d, const float* params, TcPack& pk, cudaStream_t st) {
-  if (pk.precision == HM_PREC_FP8_E4M3) {
-    tc_scales_kernel<<<pk.n_layers + 1, 256, 0, st>>>(d, params, pk.n_layers, pk.scales);
-    HM_CHECK_LAUNCH("tc_scales_kernel");
-  }
+  TcPackArgs a;
+  memset(&a, 0, sizeof(a));
+  a.d = d;
+  a.params = params;
+  a.n_layers = pk.n_layers;
+  a.blob = pk.blob;
+  a.blob_t = pk.blob_t;
+  a.scales = pk.scales;
+  uint32_t* amax = reinterpret_cast<uint32_t*>(pk.scales + 16);
+  a.amax = amax;
+  int64_t most = 1;
   for (int l = 0; l < pk.n_layers; ++l) {
-    const int64_t cnt = (int64_t)pk.N[l] * pk.K[l];
-    const int blocks = (int)((cnt + 255) / 256);
-    if (pk.precision == HM_PREC_FP8_E4M3)
-      tc_pack_kernel<TC_E4M3><<<blocks, 256, 0, st>>>(d, params, l, pk.N[l], pk.K[l], pk.boff[l], pk.scales, pk.blob);
-    else if (pk.precision == HM_PREC_BF16)
-      tc_pack_kernel<TC_BF16><<<blocks, 256, 0, st>>>(d, params, l, pk.N[l], pk.K[l], pk.boff[l], pk.scales, pk.blob);
-    else
-      tc_pack_kernel<TC_FP16><<<blocks, 256, 0, st>>>(d, params, l, pk.N[l], pk.K[l], pk.boff[l], pk.scales, pk.blob);
-    HM_CHECK_LAUNCH("tc_pack_kernel");
-    if (pk.blob_t) {
-      const int64_t ct = (int64_t)pk.NT[l] * pk.KT[l];
-      const int bt = (int)((ct + 255) / 256);
-      if (pk.precision == HM_PREC_BF16)
-        tc_pack_t_kernel<TC_BF16><<<bt, 256, 0, st>>>(d, params, l, pk.NT[l], pk.KT[l], pk.boff_t[l], pk.blob_t);
-      else
-        tc_pack_t_kernel<TC_FP16><<<bt, 256, 0, st>>>(d, params, l, pk.NT[l], pk.KT[l], pk.boff_t[l], pk.blob_t);
-      HM_CHECK_LAUNCH("tc_pack_t_kernel");
-    }
+    a.N[l] = pk.N[l];
+    a.K[l] = pk.K[l];
+    a.boff[l] = pk.boff[l];
+    a.NT[l] = pk.NT[l];
+    a.KT[l] = pk.KT[l];
+    a.boff_t[l] = pk.boff_t[l];
+    most = std::max(most, (int64_t)pk.N[l] * pk.K[l]);
   }
+  if (pk.precision == HM_PREC_FP8_E4M3) {
+    cudaError_t e = cudaMemsetAsync(amax, 0, 16 * sizeof(uint32_t), st);
+    if (e != cudaSuccess) return hm_cuda_status(e, "weight scales");
+    // encoding parameters: 64 blocks (one block of 256 threads took 0.3 ms for
+    // the renderer's million)
+    tc_amax_kernel<<<dim3(64, pk.n_layers + (d.n_enc_params > 0 ? 1 : 0)), 256, 0, st>>>(d, params, pk.n_layers, amax);
+    HM_CHECK_LAUNCH("tc_amax_kernel");
+  }
+  const dim3 grid((unsigned)((most + 255) / 256), (unsigned)pk.n_layers, pk.blob_t ? 2 : 1);
+  if (pk.precision == HM_PREC_FP8_E4M3)
+    tc_pack_kernel<TC_E4M3><<<grid, 256, 0, st>>>(a);
+  else if (pk.precision == HM_PREC_BF16)
+    tc_pack_kernel<TC_BF16><<<grid, 256, 0, st>>>(a);
+  else
+    tc_pack_kernel<TC_FP16><<<grid, 256, 0, st>>>(a);
+  HM_CHECK_LAUNCH("tc_pack_kernel");
   return HM_OK;
 }
 
