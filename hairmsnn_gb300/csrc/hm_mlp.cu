@@ -2,8 +2,9 @@
 //
 // Per batch:
 //   encode_kernel      inputs [n][in_ch] -> encoded X [n][in_pad] (pad = 1)
-//   mlp_fwd_kernel     fused: all layers of a 64-query tile in shared memory,
-//                      register-blocked SIMT GEMMs; optionally stores every
+//   mlp_x3_kernel      inference: the layers on the tensor cores (hm_mlp_x3.cu)
+//   mlp_fwd_kernel     training: all layers of a 64-query tile in shared
+//                      memory, register-blocked SIMT GEMMs; stores every
 //                      hidden activation for the backward pass
 //   mlp_bwd_kernel     fused: loss gradient + back-propagation of one tile,
 //                      stores dZ of every layer (and dX when the encoding
@@ -182,7 +183,9 @@ MlpConfig mlp_config_from_json(const char* text, int in_ch, int out_ch) {
 // Bound by the corner gathers' latency and L2 sectors (hash grids) or by the
 // sines and edges (Frequency / OneBlob).  One thread per query, writing its
 // own row, took 278 us for 262,144 queries of the hash-grid network and
-// 113 us for 517 of them (128 dependent gathers one after another).
+// 113 us for 517 of them (128 dependent gathers one after another); now 97 and
+// 7 us (whole calls at four / five / six blocks per SM: 162 / 156 / 177 us).  Loading the two corners
+// of an aligned pair of entries as one 16 bytes changed nothing.
 constexpr int kEncRows = 32;
 constexpr int kEncThreads = 256;
 
@@ -191,12 +194,14 @@ constexpr int kEncThreads = 256;
 // bins away from x's (circularly) are exactly 0 (both edges' terms are
 // clamped to the same 0 or 1) and are not evaluated.
 HM_D void oneblob_row(float x, int n_bins, float* o) {
-  const float nb = (float)n_bins;
+  const float nb = (float)n_bins, inv_nb = 1.f / nb;
+  const bool pow2 = (n_bins & (n_bins - 1)) == 0;  // then b * inv_nb is b / nb exactly
+  auto edge = [&](int b) { return pow2 ? (float)b * inv_nb : (float)b / nb; };
   const float c0 = oneblob_cdf(0.f, x, nb);
   if (n_bins <= 5 || !(x >= 0.f && x < 1.f)) {
     float left = c0;
     for (int b = 0; b < n_bins; ++b) {
-      const float right = (b == n_bins - 1) ? c0 + 1.f : oneblob_cdf((float)(b + 1) / nb, x, nb);
+      const float right = (b == n_bins - 1) ? c0 + 1.f : oneblob_cdf(edge(b + 1), x, nb);
       o[b] = right - left;
       left = right;
     }
@@ -205,11 +210,11 @@ HM_D void oneblob_row(float x, int n_bins, float* o) {
   for (int b = 0; b < n_bins; ++b) o[b] = 0.f;
   int b = min((int)(x * nb), n_bins - 1) - 2;
   b += b < 0 ? n_bins : 0;
-  float left = b == 0 ? c0 : oneblob_cdf((float)b / nb, x, nb);
+  float left = b == 0 ? c0 : oneblob_cdf(edge(b), x, nb);
 #pragma unroll 1
   for (int t = 0; t < 5; ++t) {
     const bool last = b == n_bins - 1;
-    const float right = last ? c0 + 1.f : oneblob_cdf((float)(b + 1) / nb, x, nb);
+    const float right = last ? c0 + 1.f : oneblob_cdf(edge(b + 1), x, nb);
     o[b] = right - left;
     left = last ? c0 : right;
     b = last ? 0 : b + 1;
@@ -253,7 +258,7 @@ HM_D void grid_level(const EncSeg& s, int l, const float* __restrict__ table, fl
   }
 }
 
-__global__ void __launch_bounds__(kEncThreads) encode_kernel(const __grid_constant__ MlpDims d,
+__global__ void __launch_bounds__(kEncThreads, 5) encode_kernel(const __grid_constant__ MlpDims d,
                                                              const float* __restrict__ in,
                                                              const float* __restrict__ enc_params,
                                                              float* __restrict__ X, int64_t n) {
@@ -296,11 +301,8 @@ __global__ void __launch_bounds__(kEncThreads) encode_kernel(const __grid_consta
   }
   for (int k = d.n_enc + warp; k < d.in_pad; k += kWarps) row[k] = 1.f;
   __syncthreads();
-  float* dst = X + q0 * d.in_pad;
-  for (int i = threadIdx.x; i < nq * d.in_pad; i += kEncThreads) {
-    const int q = i / d.in_pad;
-    dst[i] = rows[i + q * (ld - d.in_pad)];
-  }
+  for (int q = threadIdx.x >> 5; q < nq; q += kWarps)
+    for (int k = lane; k < d.in_pad; k += 32) X[(q0 + q) * d.in_pad + k] = rows[q * ld + k];
 }
 
 // Hash-grid gradients are scattered as 64-bit fixed-point integers (2^-40
@@ -746,8 +748,8 @@ struct Mlp {
   int step = 0;
   float lr = 0.f;
   // workspace sized for `cap` queries
-  int64_t cap = 0;
-  float* X = nullptr;        // [cap][in_pad]
+  int64_t cap = 0, x_cap = 0;
+  float* X = nullptr;        // [x_cap][in_pad] encoded inputs
   float* acts = nullptr;     // [L][cap][W]
   float* pred = nullptr;     // [cap][16]
   float* dz = nullptr;       // [L][cap][W] + [cap][16]
@@ -762,6 +764,7 @@ struct Mlp {
   // tensor-core inference (precision != FP32): packed weights, refreshed
   // when the FP32 master parameters change (params_version)
   TcPack tc;
+  uint8_t* x3_blob = nullptr;  // FP32 handles: the weights as three BF16 planes (inference)
   int64_t params_version = 1, packed_version = 0;
   int* tc_err_host = nullptr;  // host-mapped timeout flag of the kernel
   int* tc_err_dev = nullptr;
@@ -779,24 +782,36 @@ struct Mlp {
 using namespace hm;
 
 static void free_ws(Mlp* m) {
-  cudaFree(m->X);
   cudaFree(m->acts);
   cudaFree(m->pred);
   cudaFree(m->dz);
   cudaFree(m->dX);
   cudaFree(m->loss_part);
-  m->X = m->acts = m->pred = m->dz = m->dX = m->loss_part = nullptr;
+  m->acts = m->pred = m->dz = m->dX = m->loss_part = nullptr;
   m->cap = 0;
 }
 
+// Inference needs the encoded inputs alone.
+static int ensure_x(Mlp* m, int64_t n) {
+  if (n <= m->x_cap) return HM_OK;
+  cudaFree(m->X);
+  m->X = nullptr;
+  m->x_cap = 0;
+  const int64_t cap = std::max<int64_t>(n, 1024);
+  cudaError_t e = cudaMalloc(&m->X, cap * m->cfg.d.in_pad * sizeof(float));
+  if (e != cudaSuccess) return hm_cuda_status(e, "mlp encoded inputs");
+  m->x_cap = cap;
+  return HM_OK;
+}
+
 static int ensure_ws(Mlp* m, int64_t n) {
+  if (int s = ensure_x(m, n)) return s;
   if (n <= m->cap) return HM_OK;
   free_ws(m);
   const MlpDims& d = m->cfg.d;
   int64_t cap = std::max<int64_t>(n, 1024);
   cap = (cap + BM - 1) / BM * BM;
   cudaError_t e = cudaSuccess;
-  e = cudaMalloc(&m->X, cap * d.in_pad * sizeof(float));
   if (e == cudaSuccess) e = cudaMalloc(&m->acts, (int64_t)d.n_hidden * cap * d.width * sizeof(float));
   if (e == cudaSuccess) e = cudaMalloc(&m->pred, cap * 16 * sizeof(float));
   if (e == cudaSuccess) e = cudaMalloc(&m->dz, ((int64_t)d.n_hidden * cap * d.width + cap * 16) * sizeof(float));
@@ -842,6 +857,7 @@ static int launch_bwd(Mlp* m, const float* target, int loss, int64_t n, cudaStre
   return HM_OK;
 }
 
+// Training forward (SIMT, keeping the activations).
 static int dispatch_fwd(Mlp* m, const float* X, float* out, int out_stride, float* acts, int64_t n, cudaStream_t st) {
   switch (m->cfg.d.width) {
     case 16: return launch_fwd<16>(m, X, out, out_stride, acts, n, st);
@@ -948,16 +964,15 @@ extern "C" hm_mlp* hm_mlp_create(const char* config_json, int in_ch, int out_ch,
   if (e == cudaSuccess) e = cudaMalloc(&m->adam_m, bytes);
   if (e == cudaSuccess) e = cudaMalloc(&m->adam_v, bytes);
   if (e == cudaSuccess) e = cudaMalloc(&m->loss_dev, sizeof(float));
+  if (e == cudaSuccess) e = cudaHostAlloc(&m->tc_err_host, sizeof(int), cudaHostAllocMapped);
+  if (e == cudaSuccess) {
+    *m->tc_err_host = 0;
+    e = cudaHostGetDevicePointer(&m->tc_err_dev, m->tc_err_host, 0);
+  }
+  if (e == cudaSuccess && precision == HM_PREC_FP32) e = cudaMalloc(&m->x3_blob, x3_pack_bytes(m->cfg.d));
   if (e == cudaSuccess && precision != HM_PREC_FP32) {
-    e = cudaHostAlloc(&m->tc_err_host, sizeof(int), cudaHostAllocMapped);
-    if (e == cudaSuccess) {
-      *m->tc_err_host = 0;
-      e = cudaHostGetDevicePointer(&m->tc_err_dev, m->tc_err_host, 0);
-    }
-    if (e == cudaSuccess) {
-      int st = tc_pack_alloc(m->cfg.d, precision, &m->tc);
-      if (st != HM_OK) e = cudaErrorMemoryAllocation;
-    }
+    int st = tc_pack_alloc(m->cfg.d, precision, &m->tc);
+    if (st != HM_OK) e = cudaErrorMemoryAllocation;
     m->tc_train = tc_trainable(m->cfg.d, precision);
     // FP16 operands in the backward pass (FP16 handles; E4M3 handles' backward)
     m->loss_scale = precision == HM_PREC_FP16 || precision == HM_PREC_FP8_E4M3 ? 128.f : 1.f;
@@ -986,6 +1001,7 @@ extern "C" void hm_mlp_destroy(hm_mlp* h) {
   Mlp* m = (Mlp*)h;
   if (!m) return;
   free_ws(m);
+  cudaFree(m->X);
   cudaFree(m->params);
   cudaFree(m->grads);
   cudaFree(m->grads_out);
@@ -994,6 +1010,7 @@ extern "C" void hm_mlp_destroy(hm_mlp* h) {
   cudaFree(m->dw_part);
   cudaFree(m->loss_dev);
   cudaFree(m->grid_acc);
+  cudaFree(m->x3_blob);
   tc_pack_free(&m->tc);
   tc_train_free(&m->tcb);
   cudaFree(m->tc_work);
@@ -1108,6 +1125,18 @@ static int tc_inference(Mlp* m, const float* d_in, float* d_out, int64_t n, cuda
                     m->tc_err_dev, st, allow_alloc ? m->tc_work : nullptr, allow_alloc ? m->tc_work_cap : 0);
 }
 
+// FP32 inference: X [n][in_pad] holds the encoded queries' scratch.
+static int fp32_inference(Mlp* m, const float* d_in, float* X, float* d_out, int64_t n, cudaStream_t st) {
+  if (int s = tc_prepare(m)) return s;
+  const MlpDims& d = m->cfg.d;
+  if (m->packed_version != m->params_version) {
+    if (int s = x3_pack(d, m->params, m->x3_blob, st)) return s;
+    m->packed_version = m->params_version;
+  }
+  if (int s = encode(m, d_in, X, n, st)) return s;
+  return x3_forward(d, m->params, m->x3_blob, X, d_out, d.out_ch, n, m->tc_err_dev, st);
+}
+
 static int check_io(const char* who, Mlp* m, const void* a, const void* b, int64_t n) {
   if (!m) return hm_set_error("%s: NULL handle", who), HM_EINVAL;
   if (n < 0) return hm_set_error("%s: n < 0", who), HM_EINVAL;
@@ -1124,9 +1153,8 @@ extern "C" int hm_mlp_inference(hm_mlp* h, const float* d_in, float* d_out, int6
   if (n == 0) return HM_OK;
   cudaStream_t st = (cudaStream_t)stream;
   if (m->precision != HM_PREC_FP32) return tc_inference(m, d_in, d_out, n, st, true);
-  if (int s = ensure_ws(m, n)) return s;
-  if (int s = encode(m, d_in, m->X, n, st)) return s;
-  return dispatch_fwd(m, m->X, d_out, m->cfg.d.out_ch, nullptr, n, st);
+  if (int s = ensure_x(m, n)) return s;
+  return fp32_inference(m, d_in, m->X, d_out, n, st);
 }
 
 // Training forward: keeps the activations for hm_mlp_backward; d_out may be NULL.
@@ -1571,6 +1599,5 @@ extern "C" int hm_mlp_inference_noalloc(hm_mlp* h, const float* d_in, float* d_o
   float* X = nullptr;
   if (int s = noalloc_scratch(&X)) return s;
   cudaStream_t st = (cudaStream_t)stream;
-  if (int s = encode(m, d_in, X, n, st)) return s;
-  return dispatch_fwd(m, X, d_out, m->cfg.d.out_ch, nullptr, n, st);
+  return fp32_inference(m, d_in, X, d_out, n, st);
 }

@@ -171,6 +171,14 @@ struct WgradSum {
 int wgrad_sum(const WgradSum& r, const float* part, float* grads, const float* loss_part, int n_loss, float* loss_out,
               cudaStream_t st);
 
+// ---- FP32 inference on the tensor cores (hm_mlp_x3.cu): the layers of n
+// encoded queries X [n][in_pad] (16-byte aligned), weights packed as three
+// BF16 planes (x3_pack_bytes(d) bytes, repacked when the parameters change).
+int64_t x3_pack_bytes(const MlpDims& d);
+int x3_pack(const MlpDims& d, const float* params, uint8_t* blob, cudaStream_t st);
+int x3_forward(const MlpDims& d, const float* params, const uint8_t* blob, const float* X, float* out, int out_stride, int64_t n,
+               int* err_flag, cudaStream_t st);
+
 // ---- tensor-core (tcgen05) forward for HM_PREC_FP16 / BF16 / FP8_E4M3
 // Weights are repacked from the FP32 master copy into the operand layout of
 // the MMA (K-major, 8-row x 16-byte core matrices) whenever they change.
