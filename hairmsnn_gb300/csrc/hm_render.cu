@@ -116,6 +116,7 @@ constexpr int kStragglersClosest = 12;  // ... extension rays
 constexpr int kParkAnyHit = 2;        // leaves a lane parks before the leaf phase: shadow rays
 constexpr int kParkClosest = 2;       // ... extension rays
 constexpr bool kAnyHitNearest = false;  // shadow rays walk the first inner child hit next (true: the nearest)
+constexpr int kMinLanes = 4;          // rays a warp takes at least when there are few
 constexpr int kMaxRounds = 1 << 22;   // per-warp round cap (~6k rounds per warp at 512x512)
 
 // COUNT: accumulate BVH nodes visited / primitives tested (and rays) into
@@ -139,10 +140,20 @@ __global__ void __launch_bounds__(128) persistent_trace_kernel(Src src, const __
   int cur = -1;
   bool exhausted = false;
   int rounds = 0;
+  // Fewer rays than lanes: spread over all warps instead of filling the first
+  // ones.  A warp's lanes wait for one another (at its leaf phases, and for
+  // the slowest), and a launch lasts as long as its slowest warp: two 160x120
+  // path-traced frames 2.90 -> 2.49 ms, four 512x512 HairMSNN frames 14.94 ->
+  // 14.25 ms, 50,001 incoherent shadow rays 433 -> 370 us.  At least
+  // kMinLanes = 4: 1 / 2 / 4 / 8 / 16 gave 4.62 / 4.77 / 4.85 / 5.03 / 5.14 ms
+  // for two 256x192 frames and 634 / 626 / 612 / 607 / 621 us for 50,001 rays.
+  const int per_warp = max(kMinLanes, min(32, (n + gridDim.x * 4 - 1) / (gridDim.x * 4)));
+  const unsigned lanes = FULL >> (32 - per_warp);
+  const int stragglers = (ANY_HIT ? kStragglersAnyHit : kStragglersClosest) * per_warp / 32;
   for (;;) {
     // refill idle lanes; a lane whose entry holds no ray (a shadow slot
     // left empty) fetches again at once instead of idling for a round
-    unsigned idle = __ballot_sync(FULL, cur < 0);
+    unsigned idle = __ballot_sync(FULL, cur < 0) & lanes;
     while (idle && !exhausted) {
       const int leader = __ffs(idle) - 1;
       const int want = __popc(idle);
@@ -152,7 +163,7 @@ __global__ void __launch_bounds__(128) persistent_trace_kernel(Src src, const __
       exhausted = base + want >= n;
       if (cur < 0) {
         const int my = base + __popc(idle & ((1u << lane) - 1u));
-        if (my < n) {
+        if (((lanes >> lane) & 1u) && my < n) {
           f3 o, d;
           if (src.ray(my, &o, &d)) {
             if (MULTI) sp = &b.scenes[b.path_scene[src.path(my)]].s;
@@ -164,7 +175,7 @@ __global__ void __launch_bounds__(128) persistent_trace_kernel(Src src, const __
           }
         }
       }
-      idle = __ballot_sync(FULL, cur < 0);
+      idle = __ballot_sync(FULL, cur < 0) & lanes;
     }
     if (exhausted && __all_sync(FULL, cur < 0)) break;
     if (++rounds > kMaxRounds) {  // safety net: never spin on a logic error
@@ -180,7 +191,7 @@ __global__ void __launch_bounds__(128) persistent_trace_kernel(Src src, const __
       const unsigned needm = __ballot_sync(FULL, need);
       if (needm == 0) break;
       const unsigned parked = __ballot_sync(FULL, cur >= 0 && t.np > 0);
-      if (parked != 0 && __popc(needm) <= (ANY_HIT ? kStragglersAnyHit : kStragglersClosest)) break;
+      if (parked != 0 && __popc(needm) <= stragglers) break;
       if (need) {
         if (ANY_HIT)
           trav_inner_step_any<COUNT, kParkAnyHit, kAnyHitNearest>(*sp, t, stack, err, &tc);
