@@ -398,6 +398,27 @@ int build_wide(Scene& sc, cudaStream_t st) {
   return status;
 }
 
+// What the traversal needs of a leaf, in one load: the first control point of
+// its segment (or ~triangle) and its primitive id.
+__global__ void __launch_bounds__(256) leaf_info_kernel(SceneDev s, const int* __restrict__ prim_of_leaf, int n,
+                                                        int2* __restrict__ out) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  const int prim = prim_of_leaf[i];
+  out[i] = make_int2(prim < s.n_hprim ? s.seg[prim % s.n_seg] : ~(prim - s.n_hprim), prim);
+}
+
+static int build_leaf_info(Scene& sc, cudaStream_t st) {
+  const int n = sc.n_prims();
+  cudaFree(sc.d_leaf_info);
+  sc.d_leaf_info = nullptr;
+  cudaError_t e = cudaMalloc(&sc.d_leaf_info, (size_t)n * sizeof(int2));
+  if (e != cudaSuccess) return hm_cuda_status(e, "bvh leaf records");
+  leaf_info_kernel<<<(n + 255) / 256, 256, 0, st>>>(sc.dev(), sc.d_prim_of_leaf, n, sc.d_leaf_info);
+  HM_CHECK_LAUNCH("leaf_info_kernel");
+  return HM_OK;
+}
+
 int Scene::build_bvh(cudaStream_t st) {
   const int n = n_prims();
   if (n <= 0) return hm_set_error("scene has no primitives"), HM_EINVAL;
@@ -415,6 +436,7 @@ int Scene::build_bvh(cudaStream_t st) {
     sd.nodes = d_nodes;
     single_leaf_kernel<<<1, 1, 0, st>>>(sd, d_nodes, d_prim_of_leaf);
     HM_CHECK_LAUNCH("single_leaf_kernel");
+    if (int s = build_leaf_info(*this, st)) return s;
     return build_wide(*this, st);
   }
   const int nb = std::min(1024, (n + 255) / 256);
@@ -452,6 +474,7 @@ int Scene::build_bvh(cudaStream_t st) {
   }
   cudaFree(bb); cudaFree(keys); cudaFree(keys_sorted); cudaFree(child);
   cudaFree(par_i); cudaFree(par_l); cudaFree(cnt); cudaFree(tmp);
+  if (status == HM_OK) status = build_leaf_info(*this, st);
   if (status == HM_OK) status = build_wide(*this, st);
   return status;
 }

@@ -677,7 +677,7 @@ int Scene::upload() {
 Scene::~Scene() {
   cudaFree(d_cp); cudaFree(d_seg); cudaFree(d_vtx); cudaFree(d_nrm); cudaFree(d_tri);
   cudaFree(d_env); cudaFree(d_cpdf); cudaFree(d_ccdf); cudaFree(d_mpdf); cudaFree(d_mcdf);
-  cudaFree(d_dlights); cudaFree(d_nodes); cudaFree(d_prim_of_leaf); cudaFree(d_wnodes);
+  cudaFree(d_dlights); cudaFree(d_nodes); cudaFree(d_prim_of_leaf); cudaFree(d_leaf_info); cudaFree(d_wnodes);
   cudaFree(d_seg_group); cudaFree(d_group_hc); cudaFree(d_group_raw);
 }
 
@@ -748,6 +748,7 @@ SceneDev Scene::dev() const {
   d.nodes = d_nodes;
   d.n_nodes = n_nodes;
   d.prim_of_leaf = d_prim_of_leaf;
+  d.leaf_info = d_leaf_info;
   d.wnodes = d_wnodes;
   d.n_wnodes = n_wnodes;
   d.has_env = has_env;

@@ -46,6 +46,7 @@ struct SceneDev {
   const float4* nodes;  // 4 float4 per node
   int n_nodes;
   const int* prim_of_leaf;  // leaf slot -> primitive id
+  const int2* leaf_info;    // leaf slot -> (first control point of its segment, or ~triangle; primitive id)
   // the same tree collapsed to kWide-wide nodes (what the traversal walks):
   // kWideF4 float4 per node, lo.x[8] hi.x[8] lo.y[8] hi.y[8] lo.z[8] hi.z[8]
   // child[8] (>= 0 wide node, < 0 leaf ~slot; empty slots: code -1 and the
@@ -128,6 +129,7 @@ struct Scene {
   float* d_dlights = nullptr;
   float4* d_nodes = nullptr;
   int* d_prim_of_leaf = nullptr;
+  int2* d_leaf_info = nullptr;
   int n_nodes = 0;
   float4* d_wnodes = nullptr;
   int n_wnodes = 0;

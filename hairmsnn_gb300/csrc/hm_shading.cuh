@@ -290,7 +290,7 @@ HM_D float4 refit_hit(const SceneDev& s, f3 ro, f3 rd, float4 hit) {
   bool ok;
   if (prim < s.n_seg) {
     const int part = clampi((int)(hit.z * (float)s.seg_split), 0, s.seg_split - 1);
-    ok = curve_intersect(s, prim, part, r, 1e30f, &t, &u);
+    ok = curve_intersect(s, __ldg(s.seg + prim), part, r, 1e30f, &t, &u);
   } else {
     ok = tri_intersect(s, prim - s.n_seg, r, 1e30f, &t, &u, &v);
   }

@@ -80,11 +80,12 @@ HM_D P4 lerp4(P4 a, P4 b, float t) {
   return P4{a.x + (b.x - a.x) * t, a.y + (b.y - a.y) * t, a.z + (b.z - a.z) * t, a.r + (b.r - a.r) * t};
 }
 
-// Part `part` of segment seg_idx (u in [part, part + 1) / s.seg_split); *u_out
+// Part `part` of a segment (u in [part, part + 1) / s.seg_split); *u_out
 // is the u of the whole segment.
-HM_D bool curve_intersect(const SceneDev& s, int seg_idx, int part, const Ray& r, float tmax, float* t_out,
+// cp0: the segment's first control point.
+HM_D bool curve_intersect(const SceneDev& s, int cp0, int part, const Ray& r, float tmax, float* t_out,
                           float* u_out) {
-  const float4* q = s.cp + __ldg(s.seg + seg_idx);
+  const float4* q = s.cp + cp0;
   const float4 q0 = __ldg(q), q1 = __ldg(q + 1), q2 = __ldg(q + 2), q3 = __ldg(q + 3);
   // B-spline -> Bezier
   const float4 w0 = make_float4((q0.x + 4.f * q1.x + q2.x) * (1.f / 6.f), (q0.y + 4.f * q1.y + q2.y) * (1.f / 6.f),
@@ -168,18 +169,22 @@ HM_D bool curve_intersect(const SceneDev& s, int seg_idx, int part, const Ray& r
   return found;
 }
 
-// A leaf primitive; *id is what the hit reports: the segment (< n_seg) or
+// A leaf (its record in s.leaf_info); *id is what the hit reports: the segment (< n_seg) or
 // n_seg + the triangle.
-HM_D bool prim_intersect(const SceneDev& s, int prim, const Ray& r, float tmax, float* t, float* u, float* v,
+HM_D bool prim_intersect(const SceneDev& s, int2 leaf, const Ray& r, float tmax, float* t, float* u, float* v,
                          int* id) {
-  if (prim < s.n_hprim) {
+  if (leaf.x >= 0) {
     *v = 0.f;
-    const int part = prim / s.n_seg;
-    *id = prim - part * s.n_seg;
-    return curve_intersect(s, *id, part, r, tmax, t, u);
+    int seg = leaf.y, part = 0;  // leaf primitive = segment + part * n_seg
+    while (seg >= s.n_seg) {
+      seg -= s.n_seg;
+      ++part;
+    }
+    *id = seg;
+    return curve_intersect(s, leaf.x, part, r, tmax, t, u);
   }
-  *id = s.n_seg + (prim - s.n_hprim);
-  return tri_intersect(s, prim - s.n_hprim, r, tmax, t, u, v);
+  *id = s.n_seg + ~leaf.x;
+  return tri_intersect(s, ~leaf.x, r, tmax, t, u, v);
 }
 
 // Work counters of a traversal (COUNT instantiations only).
@@ -250,7 +255,7 @@ struct TravState {
   int node;
   int sp;
   int visits;
-  int np;          // parked leaves (0 .. 2)
+  int np;            // parked leaves (0 .. 2)
   int pend0, pend1;  // their leaf slots
 };
 
@@ -451,11 +456,10 @@ HM_D void trav_inner_step_any(const SceneDev& s, TravState& t, int2* stack, int*
 template <bool ANY_HIT, bool COUNT>
 HM_D bool trav_leaf(const SceneDev& s, TravState& t, TraceCount* cnt) {
   for (int j = 0; j < t.np; ++j) {
-    const int prim = __ldg(s.prim_of_leaf + (j == 0 ? t.pend0 : t.pend1));
     if (COUNT) cnt->prims += 1;
     float th, u, v;
     int id;
-    if (prim_intersect(s, prim, Ray{t.o, t.d, t.tmin, t.h.t}, t.h.t, &th, &u, &v, &id)) {
+    if (prim_intersect(s, __ldg(s.leaf_info + (j == 0 ? t.pend0 : t.pend1)), Ray{t.o, t.d, t.tmin, t.h.t}, t.h.t, &th, &u, &v, &id)) {
       t.h = Hit{th, id, u, v};
       if (ANY_HIT) {
         t.np = 0;
