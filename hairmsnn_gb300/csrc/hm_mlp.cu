@@ -601,11 +601,14 @@ __global__ void __launch_bounds__(256) mlp_bwd_kernel(const __grid_constant__ Ml
 // by asynchronous copies.  8 x 16 threads: T = 64 gives each 8 x 4 sums (32
 // FMAs per three 16-byte loads; shared memory bound the kernel with 4 x 4),
 // T = 32 4 x 2, for four times the blocks where 64 would leave SMs idle.
-// Bound by FP32 issue, in small batches by the chain over a chunk; chunks of
-// 256 to 1024 queries (the longest that gives four 64 x 64 blocks per SM).
-// One launch per layer of n / 1024 blocks of 4 x 4 sums, without a ring, took
-// 3 x 104 us for 16,384 records of the hash-grid network (16 blocks each),
-// chunks of 1024 in one launch 33 us, 17 us now.
+// Bound by FP32 issue, in small batches by the chain over a chunk.  One launch
+// per layer of 4 x 4 sums, without a ring, took 3 x 104 us for 16,384 records
+// of the hash-grid network (16 blocks each), 30 us now.  Chunks of 256 would
+// take 17 us, but the length of a chunk is part of the result: Adam's first
+// steps follow a gradient's sign, and a hash-grid entry whose gradient is
+// little more than rounding takes a full step one way or the other.  Frames
+// of a cache trained with two lengths differed by up to 3e-4 of their rms.
+constexpr int kDwChunk = 1024;
 constexpr int kDwRows = 32;
 constexpr int kDwStages = 4;
 constexpr int kDwMaxLayers = 15;
@@ -1221,50 +1224,59 @@ static int mlp_backward(Mlp* m, const char* who, const float* d_target, int loss
   int dev = 0, sms = 0;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  DwArgs a;
-  memset(&a, 0, sizeof(a));
-  WgradSum r{};
-  a.n_layers = r.n_layers = d.n_hidden + 1;
-  a.n = n;
-  auto layout = [&](int T) {
-    int jobs = 0;
-    for (int l = 0; l <= d.n_hidden; ++l) {
-      a.job0[l] = jobs;
-      jobs += ((a.M[l] + T - 1) / T) * ((a.N[l] + T - 1) / T);
+  const int chunks = (int)((n + kDwChunk - 1) / kDwChunk);
+  for (int l0 = 0, l1; l0 <= d.n_hidden; l0 = l1) {
+    // layers l0 .. l1 - 1: as many as the partials' limit takes (all of them
+    // in a batch of a frame's records)
+    const int64_t begin = d.layer_off[l0];
+    auto end = [&](int l) { return l == d.n_hidden ? d.n_net_params : d.layer_off[l + 1]; };
+    for (l1 = l0 + 1; l1 <= d.n_hidden && chunks * (end(l1) - begin) <= kDwPartMax; ++l1) {
     }
-    return a.job0[d.n_hidden + 1] = jobs;
-  };
-  for (int l = 0; l <= d.n_hidden; ++l) {
-    a.M[l] = l == d.n_hidden ? d.out_pad : d.width;
-    a.N[l] = r.fan_in[l] = r.ld[l] = l == 0 ? d.in_pad : d.width;
-    a.G[l] = m->dz + (int64_t)l * n * d.width;
-    a.H[l] = l == 0 ? m->X : m->acts + (int64_t)(l - 1) * n * d.width;
-    a.poff[l] = r.poff[l] = r.goff[l] = d.layer_off[l];
+    DwArgs a;
+    memset(&a, 0, sizeof(a));
+    WgradSum r{};
+    a.n_layers = r.n_layers = l1 - l0;
+    a.n = n;
+    a.chunk = kDwChunk;
+    r.chunks = chunks;
+    auto layout = [&](int T) {
+      int jobs = 0;
+      for (int k = 0; k < a.n_layers; ++k) {
+        a.job0[k] = jobs;
+        jobs += ((a.M[k] + T - 1) / T) * ((a.N[k] + T - 1) / T);
+      }
+      return a.job0[a.n_layers] = jobs;
+    };
+    for (int l = l0; l < l1; ++l) {
+      const int k = l - l0;
+      a.M[k] = l == d.n_hidden ? d.out_pad : d.width;
+      a.N[k] = r.fan_in[k] = r.ld[k] = l == 0 ? d.in_pad : d.width;
+      a.G[k] = m->dz + (int64_t)l * n * d.width;
+      a.H[k] = l == 0 ? m->X : m->acts + (int64_t)(l - 1) * n * d.width;
+      a.poff[k] = r.poff[k] = r.goff[k] = d.layer_off[l] - begin;
+    }
+    a.stride = r.stride = r.goff[a.n_layers] = end(l1 - 1) - begin;
+    // 64 x 64 tiles where they give two blocks per SM, else 32 x 32
+    const bool wide = chunks * (int64_t)layout(64) >= 2 * (int64_t)sms;
+    if (!wide) layout(32);
+    const int64_t need = chunks * a.stride;
+    if (need > m->dw_part_cap) {
+      cudaFree(m->dw_part);
+      m->dw_part = nullptr;
+      m->dw_part_cap = 0;
+      cudaError_t e = cudaMalloc(&m->dw_part, need * sizeof(float));
+      if (e != cudaSuccess) return hm_cuda_status(e, "dw partials");
+      m->dw_part_cap = need;
+    }
+    auto kern = wide ? dw_partial_kernel<64> : dw_partial_kernel<32>;
+    const size_t sm = (size_t)kDwStages * 2 * kDwRows * ((wide ? 64 : 32) + 4) * sizeof(float);
+    cudaError_t de = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+    if (de != cudaSuccess) return hm_cuda_status(de, "dw_partial_kernel smem");
+    kern<<<dim3((unsigned)chunks, (unsigned)a.job0[a.n_layers]), kDwThreads, sm, st>>>(a, m->dw_part);
+    HM_CHECK_LAUNCH("dw_partial_kernel");
+    if (int s = wgrad_sum(r, m->dw_part, m->grads + begin, m->loss_part, (int)((n + BM - 1) / BM), m->loss_dev, st))
+      return s;
   }
-  a.stride = r.stride = r.goff[d.n_hidden + 1] = d.n_net_params;
-  // 64 x 64 tiles where chunks of 256 give two blocks per SM, else 32 x 32
-  const int jobs64 = layout(64);
-  a.chunk = 1024;
-  while (a.chunk > 256 && (n + a.chunk - 1) / a.chunk * jobs64 < 4 * (int64_t)sms) a.chunk /= 2;
-  const int chunks = r.chunks = (int)((n + a.chunk - 1) / a.chunk);
-  const bool wide = chunks * (int64_t)jobs64 >= 2 * (int64_t)sms;
-  if (!wide) layout(32);
-  const int64_t need = chunks * d.n_net_params;
-  if (need > m->dw_part_cap) {
-    cudaFree(m->dw_part);
-    m->dw_part = nullptr;
-    m->dw_part_cap = 0;
-    cudaError_t e = cudaMalloc(&m->dw_part, need * sizeof(float));
-    if (e != cudaSuccess) return hm_cuda_status(e, "dw partials");
-    m->dw_part_cap = need;
-  }
-  auto kern = wide ? dw_partial_kernel<64> : dw_partial_kernel<32>;
-  const size_t sm = (size_t)kDwStages * 2 * kDwRows * ((wide ? 64 : 32) + 4) * sizeof(float);
-  cudaError_t de = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-  if (de != cudaSuccess) return hm_cuda_status(de, "dw_partial_kernel smem");
-  kern<<<dim3((unsigned)chunks, (unsigned)a.job0[a.n_layers]), kDwThreads, sm, st>>>(a, m->dw_part);
-  HM_CHECK_LAUNCH("dw_partial_kernel");
-  if (int s = wgrad_sum(r, m->dw_part, m->grads, m->loss_part, (int)((n + BM - 1) / BM), m->loss_dev, st)) return s;
   if (d.n_enc_params > 0)
     if (int s = grid_backward(m, m->dX, n, st)) return s;
   if (d_loss) {

@@ -159,6 +159,9 @@ template <int N>
 HM_D void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
 
 // ---- sums of the weight-gradient partials (one per chunk of the batch)
+// Floats of weight-gradient partials kept at once (256 MB; a layer whose own
+// partials need more takes that): larger batches' layers go in several launches.
+constexpr int64_t kDwPartMax = (int64_t)64 << 20;
 struct WgradSum {
   int n_layers, chunks;
   int64_t goff[16];  // first gradient of each layer; [n_layers]: their number

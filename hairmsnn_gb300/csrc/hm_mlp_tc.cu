@@ -1908,62 +1908,69 @@ int tc_backward(const MlpDims& d, const TcPack& pk, const TcTrainBufs& b, const 
   };
   int tile = chunks * (int64_t)count_jobs(32) <= sms ? 32 : 64;
   while (count_jobs(tile) > kWgMaxJobs && tile < 256) tile *= 2;
-  TcWgradArgs g;
-  memset(&g, 0, sizeof(g));
-  WgradSum r{};
   const int wz = std::max(W, 16);
-  int jobs = 0, max_in = 0;
-  int64_t poff = 0;
-  for (int l = 0; l <= L; ++l) {
-    const int N = pk.N[l], K = pk.K[l];
-    for (int c = 0; c < K; c += tile) {
-      if (jobs == kWgMaxJobs) return hm_set_error("mlp: too many weight-gradient tiles"), HM_EUNSUPPORTED;
-      TcWgradJob& j = g.job[jobs++];
-      j.dz = b.dz16 + (int64_t)l * n * wz;
-      j.h = (l == 0 ? b.x16 : b.h16 + (int64_t)(l - 1) * n * W) + c;
-      j.h_pitch = l == 0 ? K : W;
-      j.n_out = N;
-      j.n_in = std::min(tile, K - c);
-      j.ld = K;
-      j.part = poff + c;
-      max_in = std::max(max_in, j.n_in);
+  for (int l0 = 0, l1; l0 <= L; l0 = l1) {
+    // layers l0 .. l1 - 1: as many as the partials' limit takes
+    auto part = [&](int l) { return (int64_t)pk.N[l] * pk.K[l]; };
+    int64_t stride = part(l0);
+    for (l1 = l0 + 1; l1 <= L && chunks * (stride + part(l1)) <= kDwPartMax; ++l1) stride += part(l1);
+    TcWgradArgs g;
+    memset(&g, 0, sizeof(g));
+    WgradSum r{};
+    int jobs = 0, max_in = 0;
+    int64_t poff = 0;
+    for (int l = l0; l < l1; ++l) {
+      const int N = pk.N[l], K = pk.K[l];
+      for (int c = 0; c < K; c += tile) {
+        if (jobs == kWgMaxJobs) return hm_set_error("mlp: too many weight-gradient tiles"), HM_EUNSUPPORTED;
+        TcWgradJob& j = g.job[jobs++];
+        j.dz = b.dz16 + (int64_t)l * n * wz;
+        j.h = (l == 0 ? b.x16 : b.h16 + (int64_t)(l - 1) * n * W) + c;
+        j.h_pitch = l == 0 ? K : W;
+        j.n_out = N;
+        j.n_in = std::min(tile, K - c);
+        j.ld = K;
+        j.part = poff + c;
+        max_in = std::max(max_in, j.n_in);
+      }
+      // the layer's weights are [out][fan_in] with fan_in <= K[l]
+      r.goff[l - l0] = d.layer_off[l] - d.layer_off[l0];
+      r.poff[l - l0] = poff;
+      r.fan_in[l - l0] = l == 0 ? d.in_pad : W;
+      r.ld[l - l0] = K;
+      poff += part(l);
     }
-    // the layer's weights are [out][fan_in] with fan_in <= K[l]
-    r.goff[l] = d.layer_off[l];
-    r.poff[l] = poff;
-    r.fan_in[l] = l == 0 ? d.in_pad : W;
-    r.ld[l] = K;
-    poff += (int64_t)N * K;
+    r.n_layers = l1 - l0;
+    r.goff[l1 - l0] = (l1 <= L ? d.layer_off[l1] : d.n_net_params) - d.layer_off[l0];
+    r.stride = stride;
+    r.chunks = chunks;
+    const int64_t need = (int64_t)chunks * stride;
+    if (need > *dw_cap) {
+      cudaFree(*dw_part);
+      *dw_part = nullptr;
+      *dw_cap = 0;
+      cudaError_t e = cudaMalloc(dw_part, need * sizeof(float));
+      if (e != cudaSuccess) return hm_cuda_status(e, "tensor-core dW partials");
+      *dw_cap = need;
+    }
+    g.dz_pitch = wz;
+    g.n = n;
+    g.chunk = kWgChunk;
+    g.part = *dw_part;
+    g.part_stride = stride;
+    g.err = err_flag;
+    g.ncols = 32;
+    while (g.ncols < max_in) g.ncols *= 2;
+    g.stage_bytes = (kTcRows / 8 + max_in / 8) * kWgGroup;
+    const size_t sm = (size_t)kWgStages * g.stage_bytes;
+    auto kern = pk.precision == HM_PREC_BF16 ? mlp_tc_wgrad_kernel<TC_BF16> : mlp_tc_wgrad_kernel<TC_FP16>;
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+    if (e != cudaSuccess) return hm_cuda_status(e, "mlp_tc_wgrad_kernel smem");
+    kern<<<dim3((unsigned)chunks, (unsigned)jobs), kTcThreads, sm, st>>>(g);
+    HM_CHECK_LAUNCH("mlp_tc_wgrad_kernel");
+    if (int s = wgrad_sum(r, *dw_part, grads + d.layer_off[l0], b.loss_part, blocks, loss_out, st)) return s;
   }
-  r.n_layers = L + 1;
-  r.goff[L + 1] = d.n_net_params;
-  r.stride = poff;
-  r.chunks = chunks;
-  const int64_t need = (int64_t)chunks * poff;
-  if (need > *dw_cap) {
-    cudaFree(*dw_part);
-    *dw_part = nullptr;
-    *dw_cap = 0;
-    cudaError_t e = cudaMalloc(dw_part, need * sizeof(float));
-    if (e != cudaSuccess) return hm_cuda_status(e, "tensor-core dW partials");
-    *dw_cap = need;
-  }
-  g.dz_pitch = wz;
-  g.n = n;
-  g.chunk = kWgChunk;
-  g.part = *dw_part;
-  g.part_stride = poff;
-  g.err = err_flag;
-  g.ncols = 32;
-  while (g.ncols < max_in) g.ncols *= 2;
-  g.stage_bytes = (kTcRows / 8 + max_in / 8) * kWgGroup;
-  const size_t sm = (size_t)kWgStages * g.stage_bytes;
-  auto kern = pk.precision == HM_PREC_BF16 ? mlp_tc_wgrad_kernel<TC_BF16> : mlp_tc_wgrad_kernel<TC_FP16>;
-  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-  if (e != cudaSuccess) return hm_cuda_status(e, "mlp_tc_wgrad_kernel smem");
-  kern<<<dim3((unsigned)chunks, (unsigned)jobs), kTcThreads, sm, st>>>(g);
-  HM_CHECK_LAUNCH("mlp_tc_wgrad_kernel");
-  return wgrad_sum(r, *dw_part, grads, b.loss_part, blocks, loss_out, st);
+  return HM_OK;
 }
 
 // ---- the bounded wait's expiry, exercised on purpose (tests)

@@ -60,3 +60,29 @@ def test_gradients_at_tile_edges(mlpmod, n, width, hidden, encoding, prec):
             assert np.abs(d).max() <= 2e-4 * np.abs(r).max(), (lo, np.abs(d).max() / np.abs(r).max())
         else:
             assert np.sqrt(np.mean(d ** 2)) <= 2.5e-2 * np.sqrt(np.mean(r ** 2)), lo
+
+
+@pytest.mark.parametrize("prec,n,encoding", [("fp32", 700001, "wide"), ("fp16", 2000001, "small")])
+def test_gradients_of_a_batch_whose_partials_go_in_several_launches(mlpmod, prec, n, encoding):
+    """More than 64 M floats of weight-gradient partials (104 k / 72 k per
+    chunk of 1024 / 2048 rows): the sum of the gradients of two parts, each in
+    one launch and cut at a chunk's end.  The partials are the same numbers;
+    three sums of at most 980 of them, mostly of one sign, err by at most
+    3 x 980 x 2^-24 = 1.8e-4 of the sum."""
+    net = mlpmod.TinyMLP(config(128, 5, encoding), 12, 3, precision=prec, seed=4)
+    gen = torch.Generator(device="cuda").manual_seed(n)
+    x = torch.rand(n, 12, generator=gen, device="cuda")
+    dy = torch.rand(n, 3, generator=gen, device="cuda") / n
+    cut = n // 4096 * 2048
+
+    def grads(rows):
+        net.forward(x[rows])
+        net.backward_output_grad(dy[rows])
+        return net.gradients().astype(np.float64)
+
+    whole = grads(slice(0, n))
+    parts = grads(slice(0, cut)) + grads(slice(cut, n))
+    for off, fo, fi in mo.Config(net.config_text, 12, 3).layer_shapes:
+        d, r = whole[off:off + fo * fi] - parts[off:off + fo * fi], whole[off:off + fo * fi]
+        assert np.abs(r).max() > 0
+        assert np.abs(d).max() <= 2e-4 * np.abs(r).max(), (off, np.abs(d).max() / np.abs(r).max())
