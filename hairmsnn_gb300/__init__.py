@@ -12,7 +12,7 @@ Nothing here computes on the CPU: a missing library raises.
 import ctypes
 
 from . import _ffi
-from ._ffi import HMError, check, hm_bsdf_queries, hm_hair_params, lib
+from ._ffi import HMError, check, hm_bsdf_queries, hm_hair_params, lib, stream_handle
 
 __all__ = ["HMError", "lib", "bsdf_eval", "bsdf_sample", "gen_bsdf_queries", "hair_params",
            "C1_HAIR"]
@@ -30,15 +30,11 @@ def _ptr(t):
         return None
     if not t.is_cuda or not t.is_contiguous():
         raise ValueError("expected a contiguous CUDA tensor")
-    return ctypes.c_void_p(t.data_ptr())
+    return t.data_ptr()
 
 
-def _stream(stream):
-    import torch
-    s = torch.cuda.current_stream() if stream is None else stream
-    return ctypes.c_void_p(s.cuda_stream)
-
-
+# A call's host time (16.6 us for bsdf_eval, 19.8 with the outputs' checks and a
+# Stream object per call) bounds batches below some 300,000 vertices.
 def bsdf_eval(wo, wi, tangent, h, hp=None, stream=None):
     """Planar float32 CUDA tensors wo/wi/tangent [3,n], h [n] -> f [3,n], pdf [n]."""
     import torch
@@ -47,7 +43,7 @@ def bsdf_eval(wo, wi, tangent, h, hp=None, stream=None):
     pdf = torch.empty((n,), dtype=torch.float32, device=h.device)
     q = hm_bsdf_queries(_ptr(wo), _ptr(wi), _ptr(tangent), _ptr(h), None)
     p = hair_params(hp)
-    check(lib().hm_bsdf_eval(ctypes.byref(q), _ptr(f), _ptr(pdf), n, ctypes.byref(p), _stream(stream)))
+    check(lib().hm_bsdf_eval(ctypes.byref(q), f.data_ptr(), pdf.data_ptr(), n, ctypes.byref(p), stream_handle(stream)))
     return f, pdf
 
 
@@ -62,8 +58,8 @@ def bsdf_eval_grad(wo, wi, tangent, h, hp=None, stream=None):
     dpdf = torch.empty((6, n), dtype=torch.float32, device=h.device)
     q = hm_bsdf_queries(_ptr(wo), _ptr(wi), _ptr(tangent), _ptr(h), None)
     p = hair_params(hp)
-    check(lib().hm_bsdf_eval_grad(ctypes.byref(q), _ptr(f), _ptr(pdf), _ptr(df), _ptr(dpdf), n, ctypes.byref(p),
-                                  _stream(stream)))
+    check(lib().hm_bsdf_eval_grad(ctypes.byref(q), f.data_ptr(), pdf.data_ptr(), df.data_ptr(), dpdf.data_ptr(), n,
+                                  ctypes.byref(p), stream_handle(stream)))
     return f, pdf, df, dpdf
 
 
@@ -76,8 +72,8 @@ def bsdf_sample(wo, tangent, h, u, hp=None, stream=None):
     pdf = torch.empty((n,), dtype=torch.float32, device=h.device)
     q = hm_bsdf_queries(_ptr(wo), None, _ptr(tangent), _ptr(h), _ptr(u))
     p = hair_params(hp)
-    check(lib().hm_bsdf_sample(ctypes.byref(q), _ptr(wi), _ptr(f), _ptr(pdf), n, ctypes.byref(p),
-                               _stream(stream)))
+    check(lib().hm_bsdf_sample(ctypes.byref(q), wi.data_ptr(), f.data_ptr(), pdf.data_ptr(), n, ctypes.byref(p),
+                               stream_handle(stream)))
     return wi, f, pdf
 
 
@@ -89,5 +85,5 @@ def gen_bsdf_queries(seed, n, device="cuda", stream=None):
     h = torch.empty((n,), **kw)
     u = torch.empty((4, n), **kw)
     check(lib().hm_bsdf_gen_queries(seed, n, _ptr(wo), _ptr(wi), _ptr(t), _ptr(h), _ptr(u),
-                                    _stream(stream)))
+                                    stream_handle(stream)))
     return wo, wi, t, h, u

@@ -107,6 +107,16 @@ def lib():
     return L
 
 
+def stream_handle(stream):
+    """The cudaStream_t of a torch stream, of the current one for None.  The
+    current stream's handle is read without making a Stream object of it (0.3
+    us a call instead of 2.9)."""
+    if stream is not None:
+        return stream.cuda_stream
+    import torch
+    return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device())
+
+
 def check(status):
     if status != 0:
         L = lib()

@@ -14,7 +14,7 @@ import os
 import numpy as np
 
 from . import _ffi
-from ._ffi import check, hm_mlp_desc, lib
+from ._ffi import check, hm_mlp_desc, lib, stream_handle
 
 CONFIG_DIR = os.path.join(os.path.dirname(os.path.abspath(__file__)), "configs")
 PRECISIONS = {"fp32": 0, "fp16": 1, "bf16": 2, "fp8": 3}
@@ -38,13 +38,7 @@ def describe(config, in_ch, out_ch):
 
 
 def _vp(t):
-    return None if t is None else ctypes.c_void_p(t.data_ptr())
-
-
-def _stream(stream):
-    import torch
-    s = torch.cuda.current_stream() if stream is None else stream
-    return ctypes.c_void_p(s.cuda_stream)
+    return None if t is None else t.data_ptr()
 
 
 class TinyMLP:
@@ -102,36 +96,36 @@ class TinyMLP:
         n = d_in.shape[0] if size is None else size
         if d_out is None:
             d_out = torch.empty((n, self.output_ch), dtype=torch.float32, device=d_in.device)
-        check(lib().hm_mlp_inference(self._h, _vp(d_in), _vp(d_out), n, _stream(stream)))
+        check(lib().hm_mlp_inference(self._h, _vp(d_in), _vp(d_out), n, stream_handle(stream)))
         return d_out
 
     def forward(self, d_in, stream=None):
         import torch
         n = d_in.shape[0]
         out = torch.empty((n, self.output_ch), dtype=torch.float32, device=d_in.device)
-        check(lib().hm_mlp_forward(self._h, _vp(d_in), _vp(out), n, _stream(stream)))
+        check(lib().hm_mlp_forward(self._h, _vp(d_in), _vp(out), n, stream_handle(stream)))
         self._last_in = d_in
         return out
 
     def backward(self, d_target, stream=None):
         import torch
         loss = torch.zeros(1, dtype=torch.float32, device=d_target.device)
-        check(lib().hm_mlp_backward(self._h, _vp(d_target), d_target.shape[0], _vp(loss), _stream(stream)))
+        check(lib().hm_mlp_backward(self._h, _vp(d_target), d_target.shape[0], _vp(loss), stream_handle(stream)))
         return loss
 
     def backward_output_grad(self, d_dy, stream=None):
         """Backward of the last forward with dL/d(output) given ([n, out_ch])."""
-        check(lib().hm_mlp_backward_output_grad(self._h, _vp(d_dy), d_dy.shape[0], _stream(stream)))
+        check(lib().hm_mlp_backward_output_grad(self._h, _vp(d_dy), d_dy.shape[0], stream_handle(stream)))
 
     def optimizer_step(self, loss_scale=1.0, stream=None):
-        check(lib().hm_mlp_optimizer_step(self._h, float(loss_scale), _stream(stream)))
+        check(lib().hm_mlp_optimizer_step(self._h, float(loss_scale), stream_handle(stream)))
 
     # trainer->training_step(input, target); trainer->loss(ctx)
     def training_step(self, d_in, d_target, stream=None, read_loss=False):
         import torch
         loss = torch.zeros(1, dtype=torch.float32, device=d_in.device)
         check(lib().hm_mlp_training_step(self._h, _vp(d_in), _vp(d_target), d_in.shape[0], _vp(loss),
-                                         _stream(stream)))
+                                         stream_handle(stream)))
         if read_loss:
             self.training_loss = float(loss.item())
         return loss

@@ -12,7 +12,7 @@ import time
 
 import numpy as np
 
-from ._ffi import check, lib
+from ._ffi import check, lib, stream_handle
 
 HM_SCENE = dict(control_points=0, segments=1, vertices=2, normals=3, triangles=4, env=5, env_cpdf=6,
                 env_ccdf=7, env_mpdf=8, env_mcdf=9, dir_lights=10, bvh_nodes=11, bvh_leaves=12, camera=13,
@@ -124,9 +124,7 @@ def _declare():
 
 
 def _stream(stream):
-    import torch
-    s = torch.cuda.current_stream() if stream is None else stream
-    return ctypes.c_void_p(s.cuda_stream)
+    return ctypes.c_void_p(stream_handle(stream))
 
 
 class Scene:
