@@ -89,7 +89,7 @@ HM_D void nrc_end_train(const NrcBufs& nb, int tr, int bounces, int hit) {
 __global__ void __launch_bounds__(128) nrc_shade_kernel(const __grid_constant__ SceneDev s, FrameParams fp,
                                                         PathState ps, FrameBufs fb, NrcBufs nb,
                                                         const int* __restrict__ queue, const int* __restrict__ count,
-                                                        int* __restrict__ keep) {
+                                                        KeepOut keep) {
   const int n = *count;
   const int P = s.width * s.height;
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
@@ -109,13 +109,13 @@ __global__ void __launch_bounds__(128) nrc_shade_kernel(const __grid_constant__ 
     if (k == 0 && !hit) {  // camera ray missed: G-buffer = Le, no cache (rayGenCam, nrc.cu:343-350)
       st4(fb.gbuf, pid, env_radiance(s, rd), 0.f);
       ps.flags[pid] = flags | F_NRC_GSNAP;
-      keep[i] = 0;
+      keep.flag[i] = 0;
       continue;
     }
     if (!hit) {  // si.hit == false after the last vertex: the path ends with beta 0
       if (train) nrc_end_train(nb, tr, k - 1, 0);
       ps.flags[pid] = flags;
-      keep[i] = 0;
+      keep.flag[i] = 0;
       continue;
     }
     const Vertex v = setup_vertex(s, ro, rd, hr);
@@ -125,7 +125,7 @@ __global__ void __launch_bounds__(128) nrc_shade_kernel(const __grid_constant__ 
       if (v.surface && v.wo_local.z < 0.f) {  // back of the head: treated as a miss, Le = 0
         st4(fb.gbuf, pid, splat(0.f), 0.f);
         ps.flags[pid] = flags | F_NRC_GSNAP;
-        keep[i] = 0;
+        keep.flag[i] = 0;
         continue;
       }
       flags |= F_PRIM_HIT;
@@ -154,7 +154,7 @@ __global__ void __launch_bounds__(128) nrc_shade_kernel(const __grid_constant__ 
           sp.x = 0.f;
         } else {
           ps.flags[pid] = flags;
-          keep[i] = 0;
+          keep.flag[i] = 0;
           continue;
         }
       } else if (spread_cond && (flags & F_NRC_SUFFIX)) {
@@ -163,7 +163,7 @@ __global__ void __launch_bounds__(128) nrc_shade_kernel(const __grid_constant__ 
         nrc_end_train(nb, tr, k - 1, 1);
         if (!(flags & F_NRC_UNBIASED)) {
           ps.flags[pid] = flags;
-          keep[i] = 0;
+          keep.flag[i] = 0;
           continue;
         }
         flags |= F_NRC_NOSPREAD;  // unbiased pixels trace on (c = 1e30)
@@ -214,7 +214,8 @@ __global__ void __launch_bounds__(128) nrc_shade_kernel(const __grid_constant__ 
     st4(ps.beta, pid, beta);
     ps.rng[pid] = rng;
     ps.flags[pid] = flags;
-    keep[i] = k_keep;
+    keep.flag[i] = k_keep;
+    if (k_keep) atomicAdd(keep.sums + i / kScanBlock, 1);
   }
 }
 
@@ -304,7 +305,7 @@ int launch_nrc_camera(const SceneDev& s, const FrameParams& fp, const PathState&
 }
 
 int launch_nrc_shade(const SceneDev& s, const FrameParams& fp, const PathState& ps, const FrameBufs& fb,
-                     const NrcBufs& nb, const int* queue, const int* count, int* keep, int grid, cudaStream_t st) {
+                     const NrcBufs& nb, const int* queue, const int* count, const KeepOut& keep, int grid, cudaStream_t st) {
   nrc_shade_kernel<<<grid, 128, 0, st>>>(s, fp, ps, fb, nb, queue, count, keep);
   HM_CHECK_LAUNCH("nrc_shade_kernel");
   return HM_OK;

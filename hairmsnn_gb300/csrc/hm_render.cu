@@ -21,7 +21,7 @@ namespace hm {
 int launch_camera(const SceneDev& s, const FrameParams& fp, const Batch& b, const PathState& ps, int* queue,
                   int* count, cudaStream_t st);
 int launch_shade(const SceneDev& s, const FrameParams& fp, const Batch& b, const PathState& ps, const FrameBufs& fb,
-                 const int* queue, const int* count, int* keep, int grid, cudaStream_t st,
+                 const int* queue, const int* count, const KeepOut& keep, int grid, cudaStream_t st,
                  const DiffParams* dp = nullptr);
 int launch_group_dual(const SceneDev& s, void* out, int n, cudaStream_t st);
 size_t group_dual_bytes();
@@ -29,7 +29,8 @@ int launch_replay_cache_grad(int P, const PathState& ps, const DiffParams& dp, f
 int launch_nrc_camera(const SceneDev& s, const FrameParams& fp, const PathState& ps, const FrameBufs& fb,
                       const NrcBufs& nb, int* queue, int* count, cudaStream_t st);
 int launch_nrc_shade(const SceneDev& s, const FrameParams& fp, const PathState& ps, const FrameBufs& fb,
-                     const NrcBufs& nb, const int* queue, const int* count, int* keep, int grid, cudaStream_t st);
+                     const NrcBufs& nb, const int* queue, const int* count, const KeepOut& keep, int grid,
+                     cudaStream_t st);
 int launch_nrc_finalize(int P, const PathState& ps, const FrameBufs& fb, float4* col_out, cudaStream_t st);
 int launch_nrc_compose(int P, int n_pix, const FrameParams& fp, const FrameBufs& fb, const NrcBufs& nb,
                        cudaStream_t st);
@@ -359,10 +360,10 @@ __global__ void grad_parts_sum_kernel(const double* __restrict__ part, int n_par
   }
 }
 
-// ---- deterministic compaction: keep[] over count entries -> next queue
-constexpr int kScanBlock = 1024;
-
-__global__ void __launch_bounds__(kScanBlock) scan_count_kernel(const int* __restrict__ keep, const int* __restrict__ count,
+// ---- deterministic compaction: the kept of count entries -> next queue
+// Block sums of keep[] for hm_queue_compact; in a frame shading makes them.
+__global__ void __launch_bounds__(kScanBlock) scan_count_kernel(const int* __restrict__ keep,
+                                                                const int* __restrict__ count,
                                                                 int* __restrict__ block_sums, int n_blocks_max) {
   const int n = *count;
   const int nb = min(n_blocks_max, (n + kScanBlock - 1) / kScanBlock);
@@ -382,68 +383,47 @@ __global__ void __launch_bounds__(kScanBlock) scan_count_kernel(const int* __res
   }
 }
 
-__global__ void scan_blocks_kernel(int* __restrict__ block_sums, const int* __restrict__ count, int* __restrict__ out_count) {
-  // single block: exclusive scan of ceil(count / kScanBlock) block sums
+// next = the entries queue[i] with keep[i] != 0, in order; *out_count their
+// number; zero[0 .. n_zero) = 0 (the sums the next round's shading adds to).
+// Each block adds up the sums before its own: at most a few thousand integers
+// from L2.  Bound by its launch; counting, scanning and scattering in three
+// launches made two 160x120 path-traced frames take 2.53 ms instead of 2.46.
+__global__ void __launch_bounds__(kScanBlock) compact_kernel(const int* __restrict__ keep,
+                                                             const int* __restrict__ queue,
+                                                             const int* __restrict__ count,
+                                                             const int* __restrict__ block_sums,
+                                                             int* __restrict__ next, int* __restrict__ out_count,
+                                                             int* __restrict__ zero, int n_zero) {
+  const unsigned FULL = 0xffffffffu;
   const int n = *count;
   const int nb = (n + kScanBlock - 1) / kScanBlock;
-  __shared__ int carry;
-  if (threadIdx.x == 0) carry = 0;
-  __syncthreads();
-  for (int base = 0; base < nb; base += blockDim.x) {
-    const int i = base + threadIdx.x;
-    int v = i < nb ? block_sums[i] : 0;
-    // inclusive warp scan
-    int x = v;
-    for (int o = 1; o < 32; o <<= 1) {
-      int y = __shfl_up_sync(0xffffffffu, x, o);
-      if ((threadIdx.x & 31) >= o) x += y;
-    }
-    __shared__ int wsum[32];
-    if ((threadIdx.x & 31) == 31) wsum[threadIdx.x >> 5] = x;
-    __syncthreads();
-    if (threadIdx.x < 32) {
-      int w = threadIdx.x < (int)(blockDim.x >> 5) ? wsum[threadIdx.x] : 0;
-      for (int o = 1; o < 32; o <<= 1) {
-        int y = __shfl_up_sync(0xffffffffu, w, o);
-        if (threadIdx.x >= o) w += y;
-      }
-      wsum[threadIdx.x] = w;
-    }
-    __syncthreads();
-    const int warp_off = (threadIdx.x >> 5) ? wsum[(threadIdx.x >> 5) - 1] : 0;
-    const int incl = x + warp_off;
-    if (i < nb) block_sums[i] = carry + incl - v;  // exclusive
-    __syncthreads();
-    if (threadIdx.x == blockDim.x - 1) carry += incl;
-    __syncthreads();
-  }
-  if (threadIdx.x == 0) *out_count = carry;
-}
-
-__global__ void __launch_bounds__(kScanBlock) scatter_kernel(const int* __restrict__ keep, const int* __restrict__ queue,
-                                                             const int* __restrict__ count,
-                                                             const int* __restrict__ block_offsets,
-                                                             int* __restrict__ next, int n_blocks_max) {
-  const int n = *count;
-  const int nb = min(n_blocks_max, (n + kScanBlock - 1) / kScanBlock);
-  __shared__ int warp_off[kScanBlock / 32];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  __shared__ int before[kScanBlock / 32], kept[kScanBlock / 32];
+  static_assert(kScanBlock == 1024, "one lane per warp of the block");
+  for (int i = blockIdx.x * kScanBlock + threadIdx.x; i < n_zero; i += gridDim.x * kScanBlock) zero[i] = 0;
+  if (nb <= 0 && blockIdx.x == 0 && threadIdx.x == 0) *out_count = 0;
+  int base = 0, done = 0;  // kept entries of the blocks before `done`
   for (int b = blockIdx.x; b < nb; b += gridDim.x) {
+    int s = 0;
+    for (int j = done + threadIdx.x; j < b; j += kScanBlock) s += block_sums[j];
     const int i = b * kScanBlock + threadIdx.x;
-    const int v = (i < n) ? keep[i] : 0;
-    const unsigned m = __ballot_sync(0xffffffffu, v != 0);
-    const int lane = threadIdx.x & 31;
-    if (lane == 0) warp_off[threadIdx.x >> 5] = __popc(m);
-    __syncthreads();
-    if (threadIdx.x == 0) {
-      int s = 0;
-      for (int w = 0; w < kScanBlock / 32; ++w) {
-        int t = warp_off[w];
-        warp_off[w] = s;
-        s += t;
-      }
+    const int v = i < n ? keep[i] : 0;
+    const unsigned m = __ballot_sync(FULL, v != 0);
+    s = __reduce_add_sync(FULL, s);
+    if (lane == 0) {
+      before[warp] = s;
+      kept[warp] = __popc(m);
     }
     __syncthreads();
-    if (v) next[block_offsets[b] + warp_off[threadIdx.x >> 5] + __popc(m & ((1u << lane) - 1u))] = queue[i];
+    const int k = kept[lane];
+    base += __reduce_add_sync(FULL, before[lane]);
+    const int off = __reduce_add_sync(FULL, lane < warp ? k : 0);
+    if (v) next[base + off + __popc(m & ((1u << lane) - 1u))] = queue[i];
+    if (b == nb - 1) {
+      const int all = __reduce_add_sync(FULL, k);
+      if (threadIdx.x == 0) *out_count = base + all;
+    }
+    done = b;
     __syncthreads();
   }
 }
@@ -541,6 +521,7 @@ struct Render {
   int last_bounces = 0;
   int sm_count = 152;
   int fetch_slots = 0;
+  int scan_blocks() const { return (P + kScanBlock - 1) / kScanBlock; }
   int blocks_extend = 0, blocks_shadow = 0;  // persistent traversal grids
   int blocks_extend_max = 0, blocks_shadow_max = 0;
   int shade_blocks_per_sm = 8;                // shading grid = SMs x this
@@ -615,14 +596,13 @@ static cudaError_t slot_alloc(Render* r, Slot& sl) {
   A4(&sl.ps.col); A4(&sl.ps.col_s); A4(&sl.ps.sh_o0); A4(&sl.ps.sh_d0); A4(&sl.ps.sh_o1);
   A4(&sl.ps.sh_d1); A4(&sl.ps.sh_c0); A4(&sl.ps.sh_c1); A4(&sl.ps.dl_w); A4(&sl.ps.dl_ws);
   A4(&sl.fb.gbuf);
-  const int nblocks = (P + kScanBlock - 1) / kScanBlock;
   if (e == cudaSuccess) e = r->alloc(&sl.q_a, P);
   if (e == cudaSuccess) e = r->alloc(&sl.q_b, P);
   if (e == cudaSuccess) e = r->alloc(&sl.keep, P);
-  if (e == cudaSuccess) e = r->alloc(&sl.block_sums, nblocks + 1);
   if (e == cudaSuccess) e = r->alloc(&sl.counts, 4);
   if (e == cudaSuccess) e = r->alloc(&sl.err, 1);
-  if (e == cudaSuccess) e = r->alloc(&sl.fetch, r->fetch_slots);
+  if (e == cudaSuccess) e = r->alloc(&sl.fetch, r->fetch_slots + 2 * r->scan_blocks());
+  sl.block_sums = sl.fetch + r->fetch_slots;
   if (e == cudaSuccess) e = r->alloc(&sl.vis, (size_t)P * 2);
   if (e == cudaSuccess) e = r->alloc(&sl.d_loss, 1);
   if (e == cudaSuccess) e = r->alloc(&sl.d_frame, 1);
@@ -863,7 +843,7 @@ static int render_frame(Render* r, cudaStream_t user, bool sync_bounces) {
   const bool counting = r->counting && sync_bounces;
   if (counting) cudaMemsetAsync(r->d_cnt, 0, 8 * sizeof(unsigned long long), st);
   const int grid = r->sm_count * r->shade_blocks_per_sm;
-  const int nblocks = (r->P + kScanBlock - 1) / kScanBlock;
+  const int nblocks = r->scan_blocks();
   int count = r->P;
   int bounces = 0;
   int64_t ext_rays = 0;
@@ -886,7 +866,9 @@ static int render_frame(Render* r, cudaStream_t user, bool sync_bounces) {
     int* q_next = sl.q_b;
     int* c_cur = sl.counts;
     int* c_next = sl.counts + 1;
-    cudaMemsetAsync(sl.fetch, 0, r->fetch_slots * sizeof(int), st);
+    int* s_cur = sl.block_sums;
+    int* s_next = sl.block_sums + r->scan_blocks();
+    cudaMemsetAsync(sl.fetch, 0, (r->fetch_slots + 2 * r->scan_blocks()) * sizeof(int), st);  // and the block sums
     mark(S_CAMERA);
     if (tfp.mode == MODE_NRC) {
       if (int e = launch_nrc_camera(sd, tfp, sl.ps, fb_trace, sl.nrc, q_cur, c_cur, st)) return e;
@@ -905,9 +887,9 @@ static int render_frame(Render* r, cudaStream_t user, bool sync_bounces) {
       if (sh != st && it > 0) cudaStreamWaitEvent(st, sl.ev_resolved, 0);
       mark(S_SHADE);
       if (tfp.mode == MODE_NRC) {
-        if (int e = launch_nrc_shade(sd, tfp, sl.ps, fb_trace, sl.nrc, q_cur, c_cur, sl.keep, grid, st)) return e;
+        if (int e = launch_nrc_shade(sd, tfp, sl.ps, fb_trace, sl.nrc, q_cur, c_cur, {sl.keep, s_cur}, grid, st)) return e;
       } else {
-        if (int e = launch_shade(sd, tfp, r->batch, sl.ps, fb_trace, q_cur, c_cur, sl.keep, grid, st)) return e;
+        if (int e = launch_shade(sd, tfp, r->batch, sl.ps, fb_trace, q_cur, c_cur, {sl.keep, s_cur}, grid, st)) return e;
       }
       mark(S_SHADOW);
       if (sh != st) {
@@ -924,11 +906,8 @@ static int render_frame(Render* r, cudaStream_t user, bool sync_bounces) {
       HM_CHECK_LAUNCH("shadow_resolve_kernel");
       if (sh != st) cudaEventRecord(sl.ev_resolved, sh);
       mark(S_COMPACT);
-      scan_count_kernel<<<std::min(nblocks, r->sm_count * 2), kScanBlock, 0, st>>>(sl.keep, c_cur, sl.block_sums,
-                                                                                    nblocks);
-      scan_blocks_kernel<<<1, 1024, 0, st>>>(sl.block_sums, c_cur, c_next);
-      scatter_kernel<<<std::min(nblocks, r->sm_count * 2), kScanBlock, 0, st>>>(sl.keep, q_cur, c_cur,
-                                                                                sl.block_sums, q_next, nblocks);
+      compact_kernel<<<std::min(nblocks, r->sm_count * 2), kScanBlock, 0, st>>>(sl.keep, q_cur, c_cur, s_cur, q_next,
+                                                                                c_next, s_next, nblocks);
       HM_CHECK_LAUNCH("compaction");
       if (sync_bounces) {
         ext_rays += count;
@@ -939,6 +918,7 @@ static int render_frame(Render* r, cudaStream_t user, bool sync_bounces) {
       }
       std::swap(q_cur, q_next);
       std::swap(c_cur, c_next);
+      std::swap(s_cur, s_next);
       ++bounces;
     }
     if (sh != st && bounces > 0) cudaStreamWaitEvent(st, sl.ev_resolved, 0);
@@ -1403,7 +1383,9 @@ static int render_pretrain(Render* r, int passes, cudaStream_t user) {
     int* q_next = sl.q_b;
     int* c_cur = sl.counts;
     int* c_next = sl.counts + 1;
-    cudaMemsetAsync(sl.fetch, 0, r->fetch_slots * sizeof(int), st);
+    int* s_cur = sl.block_sums;
+    int* s_next = sl.block_sums + r->scan_blocks();
+    cudaMemsetAsync(sl.fetch, 0, (r->fetch_slots + 2 * r->scan_blocks()) * sizeof(int), st);  // and the block sums
     const Batch nob{nullptr, nullptr, 0};
     if (int e = launch_camera(sd, fp, nob, sl.ps, q_cur, c_cur, st)) return e;
     for (int it = 0; it <= s->path_v2; ++it) {
@@ -1411,21 +1393,19 @@ static int render_pretrain(Render* r, int passes, cudaStream_t user) {
                                                        sl.fetch + 2 * it, sl.err, r->d_cnt, false,
                                                        r->blocks_extend, st))
         return e;
-      if (int e = launch_shade(sd, fp, nob, sl.ps, sl.fb, q_cur, c_cur, sl.keep, grid, st)) return e;
+      if (int e = launch_shade(sd, fp, nob, sl.ps, sl.fb, q_cur, c_cur, {sl.keep, s_cur}, grid, st)) return e;
       if (int e = launch_persistent<ShadowRays, true>(ShadowRays{sl.ps, q_cur, c_cur, sl.vis}, sd, nob, 0.f, 1e30f,
                                                       sl.fetch + 2 * it + 1, sl.err, r->d_cnt + 3, false,
                                                       r->blocks_shadow, st))
         return e;
       shadow_resolve_kernel<false><<<grid, 256, 0, st>>>(sl.ps, q_cur, c_cur, sl.vis, DiffParams{}, nullptr,
                                                          nullptr, fp.log);
-      scan_count_kernel<<<std::min(nblocks, r->sm_count * 2), kScanBlock, 0, st>>>(sl.keep, c_cur, sl.block_sums,
-                                                                                    nblocks);
-      scan_blocks_kernel<<<1, 1024, 0, st>>>(sl.block_sums, c_cur, c_next);
-      scatter_kernel<<<std::min(nblocks, r->sm_count * 2), kScanBlock, 0, st>>>(sl.keep, q_cur, c_cur,
-                                                                                sl.block_sums, q_next, nblocks);
+      compact_kernel<<<std::min(nblocks, r->sm_count * 2), kScanBlock, 0, st>>>(sl.keep, q_cur, c_cur, s_cur, q_next,
+                                                                                c_next, s_next, nblocks);
       HM_CHECK_LAUNCH("pretrain bounce");
       std::swap(q_cur, q_next);
       std::swap(c_cur, c_next);
+      std::swap(s_cur, s_next);
     }
     if (int e = launch_finalize(sd, fp, nob, sl.ps, sl.fb, st)) return e;
     if (r->have_mlp_ev) cudaStreamWaitEvent(st, r->ev_mlp, 0);
@@ -1536,34 +1516,34 @@ static int replay_frame(Render* r, int f, const float* adjoint) {
   const DiffParams dp{r->diff_col + (size_t)f * r->P, adjoint, 1.f / (float)r->diff_frames, sl.gacc, sl.stash,
                       (const HairConstsD*)r->diff_dual, r->P};
   cudaMemsetAsync(sl.gacc, 0, (size_t)rows * r->P * sizeof(float), st);
-  cudaMemsetAsync(sl.fetch, 0, r->fetch_slots * sizeof(int), st);
+  cudaMemsetAsync(sl.fetch, 0, (r->fetch_slots + 2 * r->scan_blocks()) * sizeof(int), st);  // and the block sums
   int* q_cur = sl.q_a;
   int* q_next = sl.q_b;
   int* c_cur = sl.counts;
   int* c_next = sl.counts + 1;
+  int* s_cur = sl.block_sums;
+  int* s_next = sl.block_sums + r->scan_blocks();
   if (int e = launch_camera(sd, fp, r->batch, sl.ps, q_cur, c_cur, st)) return e;
   const int grid = r->sm_count * r->shade_blocks_per_sm;
-  const int nblocks = (r->P + kScanBlock - 1) / kScanBlock;
+  const int nblocks = r->scan_blocks();
   const int rounds = bounce_rounds(r, fp);
   for (int it = 0; it < rounds; ++it) {
     if (int e = launch_persistent<ExtendRays, false>(ExtendRays{sl.ps, q_cur, c_cur}, sd, r->batch, 0.f, 1e30f,
                                                      sl.fetch + 2 * it, sl.err, r->d_cnt, false, r->blocks_extend,
                                                      st))
       return e;
-    if (int e = launch_shade(sd, fp, r->batch, sl.ps, fb, q_cur, c_cur, sl.keep, grid, st, &dp)) return e;
+    if (int e = launch_shade(sd, fp, r->batch, sl.ps, fb, q_cur, c_cur, {sl.keep, s_cur}, grid, st, &dp)) return e;
     if (int e = launch_persistent<ShadowRays, true>(ShadowRays{sl.ps, q_cur, c_cur, sl.vis}, sd, r->batch, 0.f, 1e30f,
                                                     sl.fetch + 2 * it + 1, sl.err, r->d_cnt + 3, false,
                                                     r->blocks_shadow, st))
       return e;
     shadow_resolve_kernel<true><<<grid, 256, 0, st>>>(sl.ps, q_cur, c_cur, sl.vis, dp);
-    scan_count_kernel<<<std::min(nblocks, r->sm_count * 2), kScanBlock, 0, st>>>(sl.keep, c_cur, sl.block_sums,
-                                                                                  nblocks);
-    scan_blocks_kernel<<<1, 1024, 0, st>>>(sl.block_sums, c_cur, c_next);
-    scatter_kernel<<<std::min(nblocks, r->sm_count * 2), kScanBlock, 0, st>>>(sl.keep, q_cur, c_cur, sl.block_sums,
-                                                                              q_next, nblocks);
+    compact_kernel<<<std::min(nblocks, r->sm_count * 2), kScanBlock, 0, st>>>(sl.keep, q_cur, c_cur, s_cur, q_next,
+                                                                              c_next, s_next, nblocks);
     HM_CHECK_LAUNCH("replay bounce");
     std::swap(q_cur, q_next);
     std::swap(c_cur, c_next);
+    std::swap(s_cur, s_next);
   }
   if (r->mode == MODE_MSNN)
     if (int e = launch_replay_cache_grad(r->P, sl.ps, dp, r->diff_dy + (size_t)f * r->P * 3, st)) return e;
@@ -1694,10 +1674,10 @@ extern "C" int hm_queue_compact(const int32_t* d_keep, const int32_t* d_queue, i
   if (e != cudaSuccess) return hm_cuda_status(e, "hm_queue_compact");
   const int nn = (int)n;
   cudaMemcpyAsync(buf, &nn, sizeof(int), cudaMemcpyHostToDevice, st);
-  // the launches of a bounce round's compaction (render_frame)
+  // the sums that a round's shading makes, then the round's compaction
   scan_count_kernel<<<std::min(nblocks, sms * 2), kScanBlock, 0, st>>>(d_keep, buf, buf + 2, nblocks);
-  scan_blocks_kernel<<<1, 1024, 0, st>>>(buf + 2, buf, buf + 1);
-  scatter_kernel<<<std::min(nblocks, sms * 2), kScanBlock, 0, st>>>(d_keep, d_queue, buf, buf + 2, d_out, nblocks);
+  compact_kernel<<<std::min(nblocks, sms * 2), kScanBlock, 0, st>>>(d_keep, d_queue, buf, buf + 2, d_out, buf + 1,
+                                                                    nullptr, 0);
   e = cudaGetLastError();
   int out = 0;
   if (e == cudaSuccess) e = cudaMemcpyAsync(&out, buf + 1, sizeof(int), cudaMemcpyDeviceToHost, st);

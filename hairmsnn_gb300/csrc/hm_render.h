@@ -38,6 +38,14 @@ struct NrcBufs {
 };
 
 // Structure-of-arrays path state, one slot per pixel (capacity W*H).
+// What a shading launch leaves for the queue's compaction: flag[i] = 1 if path
+// queue[i] continues, sums[i / kScanBlock] += 1 for it (sums is zero before).
+constexpr int kScanBlock = 1024;
+struct KeepOut {
+  int* __restrict__ flag;
+  int* __restrict__ sums;
+};
+
 struct PathState {
   uint32_t* rng;
   uint32_t* flags;

@@ -143,13 +143,13 @@ HM_D void replay_vertex(const HairConstsD& hcd, const Vertex& v, f3 A, f3 bw, f3
   }
 }
 
-// Shades every path of `queue`; keep[i] = 1 if path queue[i] continues.
+// Shades every path of `queue`; keep says which continue.
 // REPLAY: the same shading (same random numbers, same results) plus the
 // path-replay terms of each hair vertex (single-scene frames).
 template <bool MULTI, bool REPLAY>
 __global__ void __launch_bounds__(128) shade_kernel(const __grid_constant__ SceneDev s0, FrameParams fp, Batch b,
                                                     PathState ps, FrameBufs fb, const int* __restrict__ queue,
-                                                    const int* __restrict__ count, int* __restrict__ keep,
+                                                    const int* __restrict__ count, KeepOut keep,
                                                     DiffParams dp) {
   const int n = *count;
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
@@ -179,11 +179,11 @@ __global__ void __launch_bounds__(128) shade_kernel(const __grid_constant__ Scen
           write_cache_input(fb.nn_train_in + (size_t)rec * fp.in_ch, fp.in_ch, splat(0.f), -1.f * rd, splat(0.f));
       }
       ps.flags[pid] = flags;
-      keep[i] = 0;
+      keep.flag[i] = 0;
       continue;
     }
     if (!hit) {  // escaped after a bounce: the path ends with no contribution
-      keep[i] = 0;
+      keep.flag[i] = 0;
       continue;
     }
     Vertex v = setup_vertex(s, ro, rd, h);
@@ -294,7 +294,8 @@ __global__ void __launch_bounds__(128) shade_kernel(const __grid_constant__ Scen
     if (detached) st3(ps.beta_d, pid, beta_d);
     ps.rng[pid] = rng;
     ps.flags[pid] = flags;
-    keep[i] = k_keep;
+    keep.flag[i] = k_keep;
+    if (k_keep) atomicAdd(keep.sums + i / kScanBlock, 1);
   }
 }
 
@@ -381,7 +382,7 @@ int launch_camera(const SceneDev& s, const FrameParams& fp, const Batch& b, cons
 }
 
 int launch_shade(const SceneDev& s, const FrameParams& fp, const Batch& b, const PathState& ps, const FrameBufs& fb,
-                 const int* queue, const int* count, int* keep, int grid, cudaStream_t st, const DiffParams* dp) {
+                 const int* queue, const int* count, const KeepOut& keep, int grid, cudaStream_t st, const DiffParams* dp) {
   if (dp) {
     if (b.scenes) return hm_set_error("path replay: single-scene renders only"), HM_EINVAL;
     shade_kernel<false, true><<<grid, 128, 0, st>>>(s, fp, b, ps, fb, queue, count, keep, *dp);

@@ -449,10 +449,10 @@ int hm_render_set_instrumentation(hm_render* render, int timing, int counting);
 int hm_render_get_timings(const hm_render* render, hm_render_timings* out);
 /* The wavefront's queue compaction (no reference counterpart: the OptiX
  * megakernel has no queues): out = the entries queue[i] with keep[i] != 0,
- * in order (a stable partition), *out_count their number.  The same three
- * kernels (block counts, block-offset scan, scatter) that compact the path
- * queue between bounce rounds of a frame.  Device arrays of n int32; waits
- * for the stream. */
+ * in order (a stable partition), *out_count their number.  The kernel that
+ * compacts the path queue between bounce rounds of a frame, after one that
+ * makes the block counts (in a frame, shading does).  Device arrays of n
+ * int32; waits for the stream. */
 int hm_queue_compact(const int32_t* d_keep, const int32_t* d_queue, int64_t n, int32_t* d_out, int64_t* out_count,
                      void* stream);
 /* Per-path ray log (no reference counterpart; parity tests).  With
