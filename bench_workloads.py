@@ -994,13 +994,12 @@ class DiffBenchWorkload:
         # (bounce loop, cache adjoint, two gradient sums) + group duals, total,
         # cache forward + backward
         rounds = 3  # BETA + 1 vertices at BETA = 2
-        md = self.r.cache().info()
-        # cache forward (encode, layers) + backward (fused dgrad, loss sum,
-        # per-layer weight-gradient partials and reduction, hash-grid scatter
-        # and conversion)
-        mlp = 2 + 2 + 2 * (md.n_hidden_layers + 1) + 2
-        fwd = 1 + 7 * rounds + 1 + 2 + 1
-        rep = 1 + 7 * rounds + 3
+        # cache forward (encode, layers) + backward (fused dgrad,
+        # weight-gradient partials and their sum, hash-grid scatter and
+        # conversion)
+        mlp = 2 + 3 + 2
+        fwd = 1 + 5 * rounds + 1 + 2 + 1
+        rep = 1 + 5 * rounds + 3
         return self.spp * (fwd + rep) + 2 + mlp
 
     def units_per_step(self):
