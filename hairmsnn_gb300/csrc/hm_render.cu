@@ -806,66 +806,6 @@ __global__ void set_frame_kernel(int* d_frame, int v) { *d_frame = v; }
 // Enqueues one frame.  sync_bounces: read the queue length after every
 // bounce (instrumented frames: per-stage events, early exit); otherwise the
 // whole frame is enqueued without a host round trip.
-// ---- the traced rounds of a frame as a graph
-// Rounds 16 to 31, 32 to 63 and so on lie in conditional nodes, each inside the
-// one before, which the device skips once no path is left: a round without
-// paths still costs its chain of launches (shading, shadow rays, resolve: 7
-// us), and the host does not know how many rounds have paths.  A node that is
-// skipped costs next to nothing, one that runs 125 us, so the first comes late
-// enough that small frames do not reach it.  Two 160x120 path-traced frames
-// (12 rounds with paths of 41) / four 512x512 HairMSNN frames: 2.46 / 13.96 ms
-// without nodes, 2.53 / 14.03 with one per 4 rounds, 2.33 / 13.62 per 8, 2.35 /
-// 13.65 from 8 on in doubling steps, 2.19 / 13.78 from 16 on.
-constexpr int kFirstRounds = 16;  // even: the rounds' buffers alternate
-
-__global__ void set_condition_kernel(cudaGraphConditionalHandle h, const int* __restrict__ count) {
-  cudaGraphSetConditional(h, *count > 0 ? 1u : 0u);
-}
-
-// Appends what launch() puts on st to g, after the nodes of `end`, which
-// become the last ones of it.
-template <typename F>
-static int graph_append(cudaGraph_t g, cudaStream_t st, std::vector<cudaGraphNode_t>& end, const F& launch) {
-  cudaError_t e = cudaStreamBeginCaptureToGraph(st, g, end.data(), nullptr, end.size(), cudaStreamCaptureModeRelaxed);
-  if (e != cudaSuccess) return hm_cuda_status(e, "trace graph capture");
-  const int le = launch();
-  cudaStreamCaptureStatus status;
-  const cudaGraphNode_t* nodes = nullptr;
-  size_t n = 0;
-  const cudaError_t ie = cudaStreamGetCaptureInfo(st, &status, nullptr, nullptr, &nodes, nullptr, &n);
-  if (ie == cudaSuccess) end.assign(nodes, nodes + n);
-  cudaGraph_t same = nullptr;
-  e = cudaStreamEndCapture(st, &same);
-  if (le != HM_OK) return le;
-  if (ie != cudaSuccess) e = ie;
-  return e == cudaSuccess ? HM_OK : hm_cuda_status(e, "trace graph capture");
-}
-
-// Appends a node to g that runs *body if *count > 0.
-static int graph_append_if(cudaGraph_t g, cudaStream_t st, std::vector<cudaGraphNode_t>& end, const int* count,
-                           cudaGraph_t* body) {
-  cudaGraphConditionalHandle h;
-  cudaError_t e = cudaGraphConditionalHandleCreate(&h, g, 0, cudaGraphCondAssignDefault);
-  if (e != cudaSuccess) return hm_cuda_status(e, "trace graph condition");
-  if (int s = graph_append(g, st, end, [&] {
-        set_condition_kernel<<<1, 1, 0, st>>>(h, count);
-        HM_CHECK_LAUNCH("set_condition_kernel");
-        return (int)HM_OK;
-      }))
-    return s;
-  cudaGraphNodeParams p{};
-  p.type = cudaGraphNodeTypeConditional;
-  p.conditional.handle = h;
-  p.conditional.type = cudaGraphCondTypeIf;
-  p.conditional.size = 1;
-  cudaGraphNode_t node;
-  e = cudaGraphAddNode(&node, g, end.data(), nullptr, end.size(), &p);
-  if (e != cudaSuccess) return hm_cuda_status(e, "trace graph condition");
-  end.assign(1, node);
-  *body = p.conditional.phGraph_out[0];
-  return HM_OK;
-}
-
 static int render_frame(Render* r, cudaStream_t user, bool sync_bounces) {
   Scene* s = r->scene;
   SceneDev sd = s->dev();
@@ -921,9 +861,13 @@ static int render_frame(Render* r, cudaStream_t user, bool sync_bounces) {
   // 4.44 -> 3.02 ms, four 512x512 HairMSNN frames 22.2 -> 18.0 ms.
   // Instrumented frames run the stages one after another on one stream.
   const cudaStream_t sh = sync_bounces ? st : sl.st_shadow;
-  auto camera = [&](const FrameParams& tfp) -> int {
+  auto trace = [&](const FrameParams& tfp) -> int {
     int* q_cur = sl.q_a;
+    int* q_next = sl.q_b;
     int* c_cur = sl.counts;
+    int* c_next = sl.counts + 1;
+    int* s_cur = sl.block_sums;
+    int* s_next = sl.block_sums + r->scan_blocks();
     cudaMemsetAsync(sl.fetch, 0, (r->fetch_slots + 2 * r->scan_blocks()) * sizeof(int), st);  // and the block sums
     mark(S_CAMERA);
     if (tfp.mode == MODE_NRC) {
@@ -932,17 +876,7 @@ static int render_frame(Render* r, cudaStream_t user, bool sync_bounces) {
       if (int e = launch_camera(sd, tfp, r->batch, sl.ps, q_cur, c_cur, st)) return e;
     }
     bounces = 0;
-    return HM_OK;
-  };
-  // rounds first .. last - 1 (first even: a round's buffers alternate)
-  auto trace = [&](const FrameParams& tfp, int first, int last) -> int {
-    int* q_cur = sl.q_a;
-    int* q_next = sl.q_b;
-    int* c_cur = sl.counts;
-    int* c_next = sl.counts + 1;
-    int* s_cur = sl.block_sums;
-    int* s_next = sl.block_sums + r->scan_blocks();
-    for (int it = first; it < last && count > 0; ++it) {
+    for (int it = 0; it < rounds && count > 0; ++it) {
       cur_bounce = it;
       paths_at.push_back(count);
       mark(S_EXTEND);
@@ -950,7 +884,7 @@ static int render_frame(Render* r, cudaStream_t user, bool sync_bounces) {
                                                        sl.fetch + 2 * it, sl.err, r->d_cnt, counting,
                                                        r->blocks_extend, st))
         return e;
-      if (sh != st && it > first) cudaStreamWaitEvent(st, sl.ev_resolved, 0);
+      if (sh != st && it > 0) cudaStreamWaitEvent(st, sl.ev_resolved, 0);
       mark(S_SHADE);
       if (tfp.mode == MODE_NRC) {
         if (int e = launch_nrc_shade(sd, tfp, sl.ps, fb_trace, sl.nrc, q_cur, c_cur, {sl.keep, s_cur}, grid, st)) return e;
@@ -1004,22 +938,13 @@ static int render_frame(Render* r, cudaStream_t user, bool sync_bounces) {
       if (sl.trace_exec) cudaGraphExecDestroy(sl.trace_exec);
       sl.trace_exec = nullptr;
       cudaGraph_t g = nullptr;
-      cudaError_t e = cudaGraphCreate(&g, 0);
-      if (e != cudaSuccess) return hm_cuda_status(e, "trace graph");
-      std::vector<cudaGraphNode_t> end;  // the last nodes so far
-      int te = graph_append(g, st, end, [&] {
-        if (int x = camera(tfp)) return x;
-        return trace(tfp, 0, std::min(rounds, kFirstRounds));
-      });
-      cudaGraph_t part = g;
-      for (int it = kFirstRounds; te == HM_OK && it < rounds; it *= 2) {
-        te = graph_append_if(part, st, end, sl.counts, &part);
-        end.clear();
-        if (te == HM_OK) te = graph_append(part, st, end, [&] { return trace(tfp, it, std::min(rounds, it * 2)); });
-      }
-      if (te != HM_OK) {
-        cudaGraphDestroy(g);
-        return te;
+      cudaError_t e = cudaStreamBeginCapture(st, cudaStreamCaptureModeRelaxed);
+      if (e != cudaSuccess) return hm_cuda_status(e, "trace graph capture");
+      const int te = trace(tfp);
+      e = cudaStreamEndCapture(st, &g);
+      if (te != HM_OK || e != cudaSuccess) {
+        if (g) cudaGraphDestroy(g);
+        return te != HM_OK ? te : hm_cuda_status(e, "trace graph capture");
       }
       e = cudaGraphInstantiate(&sl.trace_exec, g, 0);
       cudaGraphDestroy(g);
@@ -1030,14 +955,12 @@ static int render_frame(Render* r, cudaStream_t user, bool sync_bounces) {
     if (e != cudaSuccess) return hm_cuda_status(e, "trace graph launch");
     bounces = rounds;
   } else {
-    if (int e = camera(fp)) return e;
-    if (int e = trace(fp, 0, rounds)) return e;
+    if (int e = trace(fp)) return e;
   }
   r->rays_extend += ext_rays;
   r->last_bounces = bounces;
   cur_bounce = -1;
-  // replayed rounds after the first ones may be skipped: not counted
-  int launches = 1 + 5 * (r->graphs && !sync_bounces ? std::min(bounces, kFirstRounds) : bounces) + 1;
+  int launches = 1 + 5 * bounces + 1;
   if (r->mode == MODE_NRC) {
     // G_BUFFER done; then inference, RENDER pass (compose + training data),
     // training step (render_nrc.cu:651-681)

@@ -438,7 +438,7 @@ int hm_render_get_stats(const hm_render* render, hm_render_stats* out);
 typedef struct hm_render_timings {
   float total_ms, camera_ms, extend_ms, shade_ms, shadow_ms, compact_ms, finalize_ms;
   float train_ms, infer_ms, compose_ms;
-  int bounces, kernel_launches; /* launches: without replayed rounds that may be skipped */
+  int bounces, kernel_launches;
   int64_t extension_rays, shadow_rays;
   int64_t extend_nodes, extend_prims, shadow_nodes, shadow_prims;
   /* per bounce (first 48): paths traced, extension and shadow traversal ms */
