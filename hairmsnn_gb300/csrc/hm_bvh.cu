@@ -399,7 +399,10 @@ int build_wide(Scene& sc, cudaStream_t st) {
 }
 
 // What the traversal needs of a leaf, in one load: the first control point of
-// its segment (or ~triangle) and its primitive id.
+// its segment (or ~triangle) and its primitive id.  8 B per leaf
+// (10 MB for 1.24 M leaves) instead of the primitive's slot, a division by the
+// number of segments and the segment, loads that depend on one another:
+// 262,144 camera rays 601 -> 590 us, 300,007 shadow rays 1076 -> 1036 us.
 __global__ void __launch_bounds__(256) leaf_info_kernel(SceneDev s, const int* __restrict__ prim_of_leaf, int n,
                                                         int2* __restrict__ out) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;

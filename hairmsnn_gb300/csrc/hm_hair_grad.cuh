@@ -24,7 +24,7 @@
 namespace hm {
 
 constexpr int kNd = 6;  // sigma_a r, g, b, beta_m, beta_n, alpha
-constexpr unsigned kSig = 1u, kBm = 8u, kBn = 16u, kAl = 32u;  // masks: sigma_a c is kSig << c
+constexpr unsigned kBm = 8u, kBn = 16u, kAl = 32u;  // masks: bits 0 to 2 are sigma_a
 
 template <unsigned M>
 struct DualT {  // partials outside M are not set

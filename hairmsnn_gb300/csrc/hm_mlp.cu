@@ -1549,8 +1549,7 @@ extern "C" int hm_mlp_describe_config(const char* config_json, int in_ch, int ou
 }
 
 // ============================================= inference without allocation
-// hm_mlp_inference_noalloc: the same encode + fused forward kernels as
-// hm_mlp_inference, but the encoded-input scratch ([n][in_pad] floats, the
+// hm_mlp_inference_noalloc: the same kernels as hm_mlp_inference, but the encoded-input scratch ([n][in_pad] floats, the
 // only per-call device memory inference needs) lives in a fixed file-scope
 // device array instead of the handle's cudaMalloc'd workspace.  It exists for
 // callers that may not allocate device memory once running: a frame loop that

@@ -459,7 +459,8 @@ HM_D bool trav_leaf(const SceneDev& s, TravState& t, TraceCount* cnt) {
     if (COUNT) cnt->prims += 1;
     float th, u, v;
     int id;
-    if (prim_intersect(s, __ldg(s.leaf_info + (j == 0 ? t.pend0 : t.pend1)), Ray{t.o, t.d, t.tmin, t.h.t}, t.h.t, &th, &u, &v, &id)) {
+    const int2 leaf = __ldg(s.leaf_info + (j == 0 ? t.pend0 : t.pend1));
+    if (prim_intersect(s, leaf, Ray{t.o, t.d, t.tmin, t.h.t}, t.h.t, &th, &u, &v, &id)) {
       t.h = Hit{th, id, u, v};
       if (ANY_HIT) {
         t.np = 0;
