@@ -920,16 +920,17 @@ __global__ void __launch_bounds__(kFzThreads, 1) mlp_tc_fused_kernel(const __gri
       const int64_t tile = blockIdx.x + k * (int64_t)gridDim.x;
       if (tile >= n_tiles) break;
       const int st = (int)(k % NS);
-      // every thread waits for the MMAs itself (a leader polling for the group
-      // costs one more barrier per layer: 300 against 120 cycles).  A thread
+      // every warp waits for the MMAs itself (a leader polling for the group
+      // costs one more barrier per layer: 300 against 120 cycles).  A warp
       // whose wait expired goes on to the group's barriers without waiting
-      // again, a leader without issuing, and the group stops at the tile's end.
+      // again, the leader's without issuing, and the group stops at the tile's
+      // end.  ok is the same in all lanes of a warp.
       bool ok = true;
       if (leader) {
         ok = mbar_wait_bounded(full + st, (uint32_t)((k / NS) & 1));
         if (ok) issue(0, smem_u32(A0 + st * p.fz_a0), K0);
       }
-      ok = ok && mbar_wait_bounded(mma_s, ph_mma);
+      ok = __all_sync(0xffffffffu, ok) && mbar_wait_warp(mma_s, ph_mma);
       if (leader && ok) mbar_arrive(empty + st);  // the stage has been read
       ph_mma ^= 1u;
       tc_fence_after();
@@ -953,7 +954,8 @@ __global__ void __launch_bounds__(kFzThreads, 1) mlp_tc_fused_kernel(const __gri
         fence_proxy_async_smem();
         group_sync(bar_id, kFzLayWarps * 32);
         if (leader && ok) issue(l, h_base, p.K[l]);
-        ok = ok && mbar_wait_bounded(mma_s, ph_mma);
+        __syncwarp();
+        ok = ok && mbar_wait_warp(mma_s, ph_mma);
         ph_mma ^= 1u;
         tc_fence_after();
       }
@@ -1008,6 +1010,7 @@ __global__ void __launch_bounds__(kFzThreads, 1) mlp_tc_fused_kernel(const __gri
     }
   }
   if (failed && lane_id == 0) atomicOr(p.err, 1);
+  __syncwarp();
   tc_fence_before();
   __syncthreads();
   tc_fence_after();

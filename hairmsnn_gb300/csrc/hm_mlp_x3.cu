@@ -271,7 +271,7 @@ __global__ void __launch_bounds__(kX3Threads, W <= 64 ? 2 : 1) mlp_x3_kernel(con
             }
         }
         publish();
-        ok = mbar_wait_bounded(&d_done, ev & 1);
+        ok = mbar_wait_warp(&d_done, ev & 1);
         ++ev;
       }
       tc_fence_after();
@@ -292,7 +292,7 @@ __global__ void __launch_bounds__(kX3Threads, W <= 64 ? 2 : 1) mlp_x3_kernel(con
           }
         }
         publish();
-        ok = mbar_wait_bounded(&d_done, ev & 1);
+        ok = mbar_wait_warp(&d_done, ev & 1);
         ++ev;
         tc_fence_after();
       }

@@ -33,14 +33,22 @@ HM_D bool mbar_wait_bounded(uint64_t* bar, uint32_t parity, uint32_t limit = kTc
     if (mbar_try_wait(bar, parity)) return true;
   return false;
 }
+// The same wait by every lane of a warp.  The lanes leave their polling loops
+// one by one; the vote brings them together again, which the tcgen05.ld or
+// whole-warp barrier that follows wants, and makes one lane's expired wait the
+// whole warp's.
+HM_D bool mbar_wait_warp(uint64_t* bar, uint32_t parity) {
+  return __all_sync(0xffffffffu, mbar_wait_bounded(bar, parity));
+}
 HM_D void fence_proxy_async_smem() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
 HM_D void mbar_arrive(uint64_t* bar) {
   asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
 }
-// Named barrier over the nthreads threads (whole warps) of one warp group,
-// returning the OR of v over them.
+// Named barrier over the nthreads threads (whole warps, converged here) of one
+// warp group, returning the OR of v over them.
 HM_D bool group_sync_or(int id, int nthreads, bool v) {
   uint32_t r;
+  __syncwarp();
   asm volatile(
       "{\n\t.reg .pred p, q;\n\t"
       "setp.ne.u32 q, %1, 0;\n\t"
@@ -51,7 +59,10 @@ HM_D bool group_sync_or(int id, int nthreads, bool v) {
       : "memory");
   return r != 0;
 }
-HM_D void group_sync(int id, int nthreads) { asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(nthreads) : "memory"); }
+HM_D void group_sync(int id, int nthreads) {
+  __syncwarp();
+  asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(nthreads) : "memory");
+}
 // The barrier's phase completes once `bytes` of asynchronous copies have
 // landed (and the one arrival of this call).
 HM_D void mbar_arrive_expect_tx(uint64_t* bar, uint32_t bytes) {
@@ -100,9 +111,11 @@ HM_D void tc_commit(uint64_t* bar) {
                : "memory");
 }
 // 16 consecutive FP32 columns of this thread's lane; the wait is in the same
-// statement so no use of the registers can be scheduled before it.
+// statement so no use of the registers can be scheduled before it.  The load is
+// a whole converged warp's, whatever branch came before it.
 HM_D void tmem_ld16(uint32_t taddr, float (&v)[16]) {
   uint32_t r[16];
+  __syncwarp();
   asm volatile(
       "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];\n\t"
       "tcgen05.wait::ld.sync.aligned;\n"
