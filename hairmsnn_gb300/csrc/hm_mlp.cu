@@ -27,6 +27,7 @@
 
 #include "hm_json.h"
 #include "hm_mlp.cuh"
+#include "hm_x3.cuh"
 
 namespace hm {
 
@@ -718,10 +719,12 @@ __global__ void __launch_bounds__(kDwThreads) dw_partial_kernel(const __grid_con
 }
 
 // Adam (tcnn semantics).  Matrix weights [0, n_matrix) get l2_reg; encoding
-// parameters with a zero gradient are left untouched (sparse update).
+// parameters with a zero gradient are left untouched (sparse update).  FP32
+// networks: a matrix weight's BF16 planes are written with it.
 __global__ void adam_kernel(float* __restrict__ w, const float* __restrict__ g, float* __restrict__ m,
                             float* __restrict__ v, int64_t n, int64_t n_matrix, float lr, float beta1,
-                            float beta2, float eps, float l2, float loss_scale) {
+                            float beta2, float eps, float l2, float loss_scale,
+                            const __grid_constant__ X3Planes planes) {
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
     float grad = g[i] / loss_scale;
     if (i >= n_matrix && grad == 0.f) continue;
@@ -729,7 +732,8 @@ __global__ void adam_kernel(float* __restrict__ w, const float* __restrict__ g, 
     if (i < n_matrix) grad += l2 * wf;
     const float m1 = m[i] = beta1 * m[i] + (1.f - beta1) * grad;
     const float v1 = v[i] = beta2 * v[i] + (1.f - beta2) * grad * grad;
-    w[i] = wf - lr / (sqrtf(v1) + eps) * m1;
+    const float next = w[i] = wf - lr / (sqrtf(v1) + eps) * m1;
+    if (i < n_matrix && planes.blob) x3_store(planes, i, next);
   }
 }
 
@@ -764,11 +768,13 @@ struct Mlp {
   long long* grid_acc = nullptr;  // fixed-point hash-grid gradient accumulator
   int64_t last_n = 0;        // batch of the last forward()
   const float* last_in = nullptr;
-  // tensor-core inference (precision != FP32): packed weights, refreshed
-  // when the FP32 master parameters change (params_version)
+  // The weights as the tensor-core kernels read them (FP32 handles: three
+  // BF16 planes).  Written with the parameters themselves, on the same stream
+  // (pack_weights and the optimizer step), so that they match wherever work is
+  // ordered after the parameters: also in a captured graph that is replayed
+  // after an optimizer step, or that holds one.
   TcPack tc;
-  uint8_t* x3_blob = nullptr;  // FP32 handles: the weights as three BF16 planes (inference)
-  int64_t params_version = 1, packed_version = 0;
+  uint8_t* x3_blob = nullptr;
   int* tc_err_host = nullptr;  // host-mapped timeout flag of the kernel
   int* tc_err_dev = nullptr;
   // FP16 / BF16 handles also train on the tensor cores; FP16 gradients carry
@@ -935,6 +941,21 @@ static void init_params(const MlpConfig& c, uint32_t seed, std::vector<float>& p
   for (int64_t i = 0; i < d.n_enc_params; ++i) p[d.n_net_params + i] = 1e-4f * (2.f * lcg_next(st) - 1.f);
 }
 
+static int pack_weights(Mlp* m, cudaStream_t st) {
+  return m->precision == HM_PREC_FP32 ? x3_pack(m->cfg.d, m->params, m->x3_blob, st)
+                                      : tc_pack(m->cfg.d, m->params, m->tc, st);
+}
+
+// The host changed the parameters: `e` is the copy's status.  Complete when it
+// returns, whatever stream uses the network next.
+static int params_written(Mlp* m, cudaError_t e, const char* who) {
+  if (e == cudaSuccess) {
+    if (int s = pack_weights(m, nullptr)) return s;
+    e = cudaStreamSynchronize(nullptr);
+  }
+  return e == cudaSuccess ? HM_OK : hm_cuda_status(e, who);
+}
+
 // ====================================================================== C ABI
 extern "C" hm_mlp* hm_mlp_create(const char* config_json, int in_ch, int out_ch, int precision,
                                  uint32_t seed, int* status) {
@@ -991,8 +1012,7 @@ extern "C" hm_mlp* hm_mlp_create(const char* config_json, int in_ch, int out_ch,
   if (e == cudaSuccess) e = cudaMemset(m->adam_m, 0, bytes);
   if (e == cudaSuccess) e = cudaMemset(m->adam_v, 0, bytes);
   if (e == cudaSuccess) e = cudaMemset(m->grads, 0, bytes);
-  if (e != cudaSuccess) {
-    *status = hm_cuda_status(e, "hm_mlp_create upload");
+  if ((*status = params_written(m, e, "hm_mlp_create upload")) != HM_OK) {
     hm_mlp_destroy((hm_mlp*)m);
     return nullptr;
   }
@@ -1051,8 +1071,7 @@ extern "C" int hm_mlp_set_params(hm_mlp* h, const float* host_in) {
   Mlp* m = (Mlp*)h;
   if (!m || !host_in) return hm_set_error("hm_mlp_set_params: NULL"), HM_EINVAL;
   cudaError_t e = cudaMemcpy(m->params, host_in, m->n_params * sizeof(float), cudaMemcpyHostToDevice);
-  m->params_version += 1;
-  return e == cudaSuccess ? HM_OK : hm_cuda_status(e, "hm_mlp_set_params");
+  return params_written(m, e, "hm_mlp_set_params");
 }
 
 extern "C" int hm_mlp_get_gradients(const hm_mlp* h, float* host_out) {
@@ -1084,8 +1103,7 @@ extern "C" int hm_mlp_reset(hm_mlp* h) {
   if (e == cudaSuccess) e = cudaMemset(m->adam_v, 0, bytes);
   m->step = 0;
   m->lr = m->cfg.adam.lr;
-  m->params_version += 1;
-  return e == cudaSuccess ? HM_OK : hm_cuda_status(e, "hm_mlp_reset");
+  return params_written(m, e, "hm_mlp_reset");
 }
 
 // A bounded tensor-core wait that expired in an earlier call is reported here.
@@ -1104,14 +1122,7 @@ static int tc_prepare(Mlp* m) {
 // the layer kernels.  A bounded wait that expired in an earlier call is
 // reported here.
 static int tc_inference(Mlp* m, const float* d_in, float* d_out, int64_t n, cudaStream_t st, bool allow_alloc) {
-  if (*(volatile int*)m->tc_err_host) {
-    *m->tc_err_host = 0;
-    return hm_set_error("mlp: a tensor-core wait expired in an earlier call"), HM_ETIMEOUT;
-  }
-  if (m->packed_version != m->params_version) {
-    if (int s = tc_pack(m->cfg.d, m->params, m->tc, st)) return s;
-    m->packed_version = m->params_version;
-  }
+  if (int s = tc_prepare(m)) return s;
   allow_alloc = allow_alloc && tc_wants_workspace(m->cfg.d, m->tc);
   if (allow_alloc) {
     const int64_t need = tc_encode_bytes(m->cfg.d, m->tc, n);
@@ -1132,10 +1143,6 @@ static int tc_inference(Mlp* m, const float* d_in, float* d_out, int64_t n, cuda
 static int fp32_inference(Mlp* m, const float* d_in, float* X, float* d_out, int64_t n, cudaStream_t st) {
   if (int s = tc_prepare(m)) return s;
   const MlpDims& d = m->cfg.d;
-  if (m->packed_version != m->params_version) {
-    if (int s = x3_pack(d, m->params, m->x3_blob, st)) return s;
-    m->packed_version = m->params_version;
-  }
   if (int s = encode(m, d_in, X, n, st)) return s;
   return x3_forward(d, m->params, m->x3_blob, X, d_out, d.out_ch, n, m->tc_err_dev, st);
 }
@@ -1172,10 +1179,6 @@ extern "C" int hm_mlp_forward(hm_mlp* h, const float* d_in, float* d_out, int64_
     if (n > m->tcb.cap) {
       const int64_t cap = std::max<int64_t>((n + 127) / 128 * 128, 1024);
       if (int s = tc_train_alloc(m->cfg.d, cap, m->cfg.d.n_enc_params > 0, &m->tcb)) return s;
-    }
-    if (m->packed_version != m->params_version) {
-      if (int s = tc_pack(m->cfg.d, m->params, m->tc, st)) return s;
-      m->packed_version = m->params_version;
     }
     if (int s = tc_train_forward(m->cfg.d, m->tc, m->params + m->cfg.d.n_net_params, d_in, n, m->tcb, m->tc_err_dev,
                                  st))
@@ -1313,10 +1316,9 @@ extern "C" int hm_mlp_optimizer_step(hm_mlp* h, float loss_scale, void* stream) 
   const float lr_t = (float)(m->lr * sqrt(1.0 - pow((double)a.beta2, t)) / (1.0 - pow((double)a.beta1, t)));
   adam_kernel<<<1024, 256, 0, (cudaStream_t)stream>>>(m->params, m->grads, m->adam_m, m->adam_v, m->n_params,
                                                       m->cfg.d.n_net_params, lr_t, a.beta1, a.beta2, a.eps,
-                                                      a.l2_reg, loss_scale);
+                                                      a.l2_reg, loss_scale, x3_planes(m->cfg.d, m->x3_blob));
   HM_CHECK_LAUNCH("adam_kernel");
-  m->params_version += 1;
-  return HM_OK;
+  return m->precision == HM_PREC_FP32 ? HM_OK : pack_weights(m, (cudaStream_t)stream);
 }
 
 // Trainer::training_step (render_hair_msnn.cu:690): forward, loss, backward,

@@ -176,7 +176,7 @@ int wgrad_sum(const WgradSum& r, const float* part, float* grads, const float* l
 
 // ---- FP32 inference on the tensor cores (hm_mlp_x3.cu): the layers of n
 // encoded queries X [n][in_pad] (16-byte aligned), weights packed as three
-// BF16 planes (x3_pack_bytes(d) bytes, repacked when the parameters change).
+// BF16 planes (x3_pack_bytes(d) bytes, written by what writes the parameters).
 int64_t x3_pack_bytes(const MlpDims& d);
 int x3_pack(const MlpDims& d, const float* params, uint8_t* blob, cudaStream_t st);
 int x3_forward(const MlpDims& d, const float* params, const uint8_t* blob, const float* X, float* out, int out_stride, int64_t n,

@@ -44,6 +44,7 @@
 
 #include "hm_mlp.cuh"
 #include "hm_tc.cuh"
+#include "hm_x3.cuh"
 
 namespace hm {
 
@@ -325,31 +326,17 @@ __global__ void __launch_bounds__(kX3Threads, W <= 64 ? 2 : 1) mlp_x3_kernel(con
   if (warp == 0) tmem_dealloc(tmem, kCols);
 }
 
-// The planes of every matrix, K step after K step: [w0 | w1 | w2] rows of one
-// 16-wide step as core matrices.
-__global__ void __launch_bounds__(256) x3_pack_kernel(const __grid_constant__ MlpDims d, const float* __restrict__ params,
-                                                      uint8_t* __restrict__ blob) {
+// The planes of every matrix (adam_kernel keeps them up to date afterwards).
+__global__ void __launch_bounds__(256) x3_pack_kernel(const __grid_constant__ X3Planes p,
+                                                      const float* __restrict__ params) {
   const int64_t i = blockIdx.x * (int64_t)256 + threadIdx.x;  // element of the matrix parameters
-  if (i >= d.n_net_params) return;
-  int l = 0;
-  while (l < d.n_hidden && i >= d.layer_off[l + 1]) ++l;
-  const int K = l == 0 ? d.in_pad : d.width, N = l == d.n_hidden ? d.out_pad : d.width;
-  const int64_t j = i - d.layer_off[l];
-  const int o = (int)(j / K), k = (int)(j % K);
-  uint8_t* step = blob + 6 * d.layer_off[l] + (int64_t)(k / 16) * (3 * N * 32);
-  float v = params[i];
-#pragma unroll
-  for (int pl = 0; pl < 3; ++pl) {
-    const __nv_bfloat16 h = __float2bfloat16_rn(v);
-    *reinterpret_cast<__nv_bfloat16*>(step + op_offset(3 * N, pl * N + o, (k % 16) * 2)) = h;
-    v -= __bfloat162float(h);
-  }
+  if (i < p.n_net_params) x3_store(p, i, params[i]);
 }
 
 int64_t x3_pack_bytes(const MlpDims& d) { return 6 * d.n_net_params; }
 
 int x3_pack(const MlpDims& d, const float* params, uint8_t* blob, cudaStream_t st) {
-  x3_pack_kernel<<<(unsigned)((d.n_net_params + 255) / 256), 256, 0, st>>>(d, params, blob);
+  x3_pack_kernel<<<(unsigned)((d.n_net_params + 255) / 256), 256, 0, st>>>(x3_planes(d, blob), params);
   HM_CHECK_LAUNCH("x3_pack_kernel");
   return HM_OK;
 }

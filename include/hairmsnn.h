@@ -120,7 +120,9 @@ int hm_bsdf_gen_queries(uint32_t seed, int64_t n, float* wo, float* wi, float* t
  * (tiny-cuda-nn's column-major GPUMatrix(ptr, ch, n)).  Any n >= 0 is
  * accepted (the reference needs n % 128 == 0, scene.cpp:300-306).  The
  * handle owns parameters, optimizer state and workspace; one handle per
- * stream at a time.
+ * stream at a time.  An inference or a training step captured in a CUDA graph
+ * (after one direct call of the same size) uses the parameters of the moment
+ * it is replayed.
  * ---------------------------------------------------------------------- */
 typedef enum hm_precision {
   HM_PREC_FP32 = 0,
