@@ -14,6 +14,7 @@ void hm_set_error(const char* fmt, ...) {
 }
 
 int hm_cuda_status(cudaError_t e, const char* what) {
+  cudaGetLastError();  // reported here: the next launch's check must not find it again
   hm_set_error("%s: %s (%s)", what, cudaGetErrorName(e), cudaGetErrorString(e));
   return e == cudaErrorMemoryAllocation ? HM_ENOMEM : HM_ECUDA;
 }
