@@ -754,9 +754,10 @@ struct Mlp {
   float* adam_v = nullptr;
   int step = 0;
   float lr = 0.f;
-  // workspace sized for `cap` queries
-  int64_t cap = 0, x_cap = 0;
-  float* X = nullptr;        // [x_cap][in_pad] encoded inputs
+  // workspace of a training step, sized for `cap` records: what the forward
+  // leaves in it is the backward's, so inference has inputs of its own
+  int64_t cap = 0;
+  float* X = nullptr;        // [cap][in_pad] encoded inputs
   float* acts = nullptr;     // [L][cap][W]
   float* pred = nullptr;     // [cap][16]
   float* dz = nullptr;       // [L][cap][W] + [cap][16]
@@ -764,9 +765,11 @@ struct Mlp {
   float* dw_part = nullptr;  // split partials
   int64_t dw_part_cap = 0;
   float* loss_part = nullptr;
+  int64_t xi_cap = 0;
+  float* Xi = nullptr;       // [xi_cap][in_pad] encoded inputs of an inference
   float* loss_dev = nullptr;
   long long* grid_acc = nullptr;  // fixed-point hash-grid gradient accumulator
-  int64_t last_n = 0;        // batch of the last forward()
+  int64_t last_n = 0;        // batch of the last forward(), 0 while its buffers hold none
   const float* last_in = nullptr;
   // The weights as the tensor-core kernels read them (FP32 handles: three
   // BF16 planes).  Written with the parameters themselves, on the same stream
@@ -791,36 +794,35 @@ struct Mlp {
 using namespace hm;
 
 static void free_ws(Mlp* m) {
+  cudaFree(m->X);
   cudaFree(m->acts);
   cudaFree(m->pred);
   cudaFree(m->dz);
   cudaFree(m->dX);
   cudaFree(m->loss_part);
-  m->acts = m->pred = m->dz = m->dX = m->loss_part = nullptr;
+  m->X = m->acts = m->pred = m->dz = m->dX = m->loss_part = nullptr;
   m->cap = 0;
 }
 
-// Inference needs the encoded inputs alone.
-static int ensure_x(Mlp* m, int64_t n) {
-  if (n <= m->x_cap) return HM_OK;
-  cudaFree(m->X);
-  m->X = nullptr;
-  m->x_cap = 0;
+static int ensure_xi(Mlp* m, int64_t n) {
+  if (n <= m->xi_cap) return HM_OK;
+  cudaFree(m->Xi);
+  m->Xi = nullptr;
+  m->xi_cap = 0;
   const int64_t cap = std::max<int64_t>(n, 1024);
-  cudaError_t e = cudaMalloc(&m->X, cap * m->cfg.d.in_pad * sizeof(float));
+  cudaError_t e = cudaMalloc(&m->Xi, cap * m->cfg.d.in_pad * sizeof(float));
   if (e != cudaSuccess) return hm_cuda_status(e, "mlp encoded inputs");
-  m->x_cap = cap;
+  m->xi_cap = cap;
   return HM_OK;
 }
 
 static int ensure_ws(Mlp* m, int64_t n) {
-  if (int s = ensure_x(m, n)) return s;
   if (n <= m->cap) return HM_OK;
   free_ws(m);
   const MlpDims& d = m->cfg.d;
   int64_t cap = std::max<int64_t>(n, 1024);
   cap = (cap + BM - 1) / BM * BM;
-  cudaError_t e = cudaSuccess;
+  cudaError_t e = cudaMalloc(&m->X, cap * d.in_pad * sizeof(float));
   if (e == cudaSuccess) e = cudaMalloc(&m->acts, (int64_t)d.n_hidden * cap * d.width * sizeof(float));
   if (e == cudaSuccess) e = cudaMalloc(&m->pred, cap * 16 * sizeof(float));
   if (e == cudaSuccess) e = cudaMalloc(&m->dz, ((int64_t)d.n_hidden * cap * d.width + cap * 16) * sizeof(float));
@@ -1024,7 +1026,7 @@ extern "C" void hm_mlp_destroy(hm_mlp* h) {
   Mlp* m = (Mlp*)h;
   if (!m) return;
   free_ws(m);
-  cudaFree(m->X);
+  cudaFree(m->Xi);
   cudaFree(m->params);
   cudaFree(m->grads);
   cudaFree(m->grads_out);
@@ -1163,8 +1165,8 @@ extern "C" int hm_mlp_inference(hm_mlp* h, const float* d_in, float* d_out, int6
   if (n == 0) return HM_OK;
   cudaStream_t st = (cudaStream_t)stream;
   if (m->precision != HM_PREC_FP32) return tc_inference(m, d_in, d_out, n, st, true);
-  if (int s = ensure_x(m, n)) return s;
-  return fp32_inference(m, d_in, m->X, d_out, n, st);
+  if (int s = ensure_xi(m, n)) return s;
+  return fp32_inference(m, d_in, m->Xi, d_out, n, st);
 }
 
 // Training forward: keeps the activations for hm_mlp_backward; d_out may be NULL.
@@ -1176,6 +1178,7 @@ extern "C" int hm_mlp_forward(hm_mlp* h, const float* d_in, float* d_out, int64_
   const float* pred = nullptr;
   if (m->tc_train) {
     if (int s = tc_prepare(m)) return s;
+    m->last_n = 0;
     if (n > m->tcb.cap) {
       const int64_t cap = std::max<int64_t>((n + 127) / 128 * 128, 1024);
       if (int s = tc_train_alloc(m->cfg.d, cap, m->cfg.d.n_enc_params > 0, &m->tcb)) return s;
@@ -1185,6 +1188,7 @@ extern "C" int hm_mlp_forward(hm_mlp* h, const float* d_in, float* d_out, int64_
       return s;
     pred = m->tcb.pred;
   } else {
+    m->last_n = 0;
     if (int s = ensure_ws(m, n)) return s;
     if (int s = encode(m, d_in, m->X, n, st)) return s;
     if (int s = dispatch_fwd(m, m->X, m->pred, 16, m->acts, n, st)) return s;
