@@ -107,18 +107,22 @@ HM_D void x3_sum16(uint32_t row_taddr, int col, bool two, float (&v)[16]) {
   for (int e = 0; e < 16; ++e) v[e] += t[e];
 }
 
-// Values whose planes could be infinite: their rows are computed again in
-// plain FP32 (x3_plain_row).
+// Rows that the planes cannot carry are computed again with multiply-adds
+// (x3_plain_row): those with an input of at least kX3Huge, and those with a sum
+// that is not finite.  An infinity or NaN among a row's inputs, activations or
+// weights, a value that rounds to infinity in BF16 (inf - inf in the next
+// plane) and a partial sum that overflows all leave such a sum; the
+// multiply-adds may have a number or an infinity there.
 constexpr float kX3Huge = 1e30f;
+// Their first output until then: a NaN that arithmetic does not produce.
+constexpr uint32_t kX3Mark = 0x7fc05a5au;
 
-// Eight values as three planes' 16-byte groups at dst + plane * a_plane; amax
-// collects their largest magnitude (a NaN passes through its planes).
-HM_D void x3_split8(const float (&v)[8], uint8_t* dst, uint32_t a_plane, float& amax) {
+// Eight values as three planes' 16-byte groups at dst + plane * a_plane.
+HM_D void x3_split8(const float (&v)[8], uint8_t* dst, uint32_t a_plane) {
   uint32_t w[3][4];
 #pragma unroll
   for (int i = 0; i < 4; ++i) {
     float x = v[2 * i], y = v[2 * i + 1];
-    amax = fmaxf(amax, fmaxf(fabsf(x), fabsf(y)));
 #pragma unroll
     for (int p = 0; p < 3; ++p) {
       const __nv_bfloat162 h = __floats2bfloat162_rn(x, y);
@@ -133,24 +137,25 @@ HM_D void x3_split8(const float (&v)[8], uint8_t* dst, uint32_t a_plane, float& 
     *reinterpret_cast<uint4*>(dst + p * a_plane) = make_uint4(w[p][0], w[p][1], w[p][2], w[p][3]);
 }
 
-// One query layer by layer with FP32 multiply-adds in input order: rows with
-// infinite or huge values, where inf - inf in the split planes would turn an
-// infinity into a NaN.
+// One query layer by layer with FP32 multiply-adds in input order, by one warp
+// (a lane has every 32nd output of a layer); h: 2 * 128 floats of the warp's.
 static __device__ __noinline__ void x3_plain_row(const MlpDims& d, const float* __restrict__ params,
-                                                 const float* __restrict__ x, float* __restrict__ out, int out_ch) {
-  float h[2][128];
+                                                 const float* __restrict__ x, float* h, float* __restrict__ out,
+                                                 int out_ch) {
+  const int lane = threadIdx.x & 31;
   for (int l = 0; l <= d.n_hidden; ++l) {
     const int K = l == 0 ? d.in_pad : d.width, N = l == d.n_hidden ? out_ch : d.width;
-    const float* src = l == 0 ? x : h[l & 1];
-    for (int o = 0; o < N; ++o) {
+    const float* src = l == 0 ? x : h + (l & 1) * 128;
+    for (int o = lane; o < N; o += 32) {
       const float* w = params + d.layer_off[l] + (int64_t)o * K;
       float acc = 0.f;
       for (int k = 0; k < K; ++k) acc = fmaf(src[k], w[k], acc);
       if (l == d.n_hidden)
         out[o] = acc;
       else
-        h[(l + 1) & 1][o] = fmaxf(acc, 0.f);
+        h[((l + 1) & 1) * 128 + o] = fmaxf(acc, 0.f);
     }
+    __syncwarp();
   }
 }
 
@@ -160,7 +165,8 @@ __global__ void __launch_bounds__(kX3Threads, W <= 64 ? 2 : 1) mlp_x3_kernel(con
   extern __shared__ __align__(1024) uint8_t smem[];
   __shared__ __align__(8) uint64_t w_full[kX3Slots], w_empty[kX3Slots], a_ready, d_done;
   __shared__ uint32_t holder;
-  __shared__ uint8_t huge[2][kTcRows];  // rows to compute in plain FP32, by tile parity
+  __shared__ uint8_t huge[2][kTcRows];  // rows for x3_plain_row, by tile parity
+  __shared__ int any_huge;
   uint8_t* A = smem;
   uint8_t* ring = smem + 3 * p.a_plane;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -175,6 +181,7 @@ __global__ void __launch_bounds__(kX3Threads, W <= 64 ? 2 : 1) mlp_x3_kernel(con
   }
   if (warp == 0) tmem_alloc(&holder, kCols);
   if (tid < 2 * kTcRows) huge[tid / kTcRows][tid % kTcRows] = 0;
+  if (tid == 0) any_huge = 0;
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
@@ -249,6 +256,7 @@ __global__ void __launch_bounds__(kX3Threads, W <= 64 ? 2 : 1) mlp_x3_kernel(con
     };
     for (int64_t tile = blockIdx.x; tile < n_tiles; tile += gridDim.x, parity ^= 1) {
       float amax = 0.f;
+      float zero = 0.f;  // NaN once a sum is not finite
       const int64_t q = tile * kTcRows + row;
       const bool valid = q < p.n;
       const float* x = p.X + (valid ? q : 0) * p.in_pad;
@@ -268,7 +276,9 @@ __global__ void __launch_bounds__(kX3Threads, W <= 64 ? 2 : 1) mlp_x3_kernel(con
             if (g0 + 2 * i < groups) {
               const float v[8] = {u[i][0].x, u[i][0].y, u[i][0].z, u[i][0].w,
                                   u[i][1].x, u[i][1].y, u[i][1].z, u[i][1].w};
-              x3_split8(v, a_row + (g0 + 2 * i) * (16 * kTcRows), p.a_plane, amax);
+#pragma unroll
+              for (int e = 0; e < 8; ++e) amax = fmaxf(amax, fabsf(v[e]));
+              x3_split8(v, a_row + (g0 + 2 * i) * (16 * kTcRows), p.a_plane);
             }
         }
         publish();
@@ -288,8 +298,11 @@ __global__ void __launch_bounds__(kX3Threads, W <= 64 ? 2 : 1) mlp_x3_kernel(con
             if (W < 32 && g != half) continue;  // W = 16: eight columns each
             float v[8];
 #pragma unroll
-            for (int e = 0; e < 8; ++e) v[e] = fmaxf(h[g * 8 + e], 0.f);
-            x3_split8(v, a_row + (col / 8 + g) * (16 * kTcRows), p.a_plane, amax);
+            for (int e = 0; e < 8; ++e) {
+              zero = __fmaf_rn(h[g * 8 + e], 0.f, zero);
+              v[e] = fmaxf(h[g * 8 + e], 0.f);
+            }
+            x3_split8(v, a_row + (col / 8 + g) * (16 * kTcRows), p.a_plane);
           }
         }
         publish();
@@ -298,7 +311,7 @@ __global__ void __launch_bounds__(kX3Threads, W <= 64 ? 2 : 1) mlp_x3_kernel(con
         tc_fence_after();
       }
       // both halves of a row have marked it; a role that failed stops the group
-      if (amax >= kX3Huge) huge[parity][row] = 1;
+      if (amax >= kX3Huge || zero != 0.f) huge[parity][row] = 1;
       if (group_sync_or(1, kX3Compute, !ok)) {
         ok = false;
         break;
@@ -306,14 +319,20 @@ __global__ void __launch_bounds__(kX3Threads, W <= 64 ? 2 : 1) mlp_x3_kernel(con
       if (half == 0) {
         float y[16];
         x3_sum16<16>(row_taddr, 0, W > 16, y);
-        const bool plain = huge[parity][row] != 0;
+        zero = huge[parity][row];
         huge[parity][row] = 0;
         if (valid) {
           float* out = p.out + q * p.out_stride;
 #pragma unroll
           for (int o = 0; o < 16; ++o)
-            if (o < p.out_ch) out[o] = y[o];
-          if (plain) x3_plain_row(p.d, p.params, x, out, p.out_ch);
+            if (o < p.out_ch) {
+              out[o] = y[o];
+              zero = __fmaf_rn(y[o], 0.f, zero);
+            }
+          if (zero != 0.f) {
+            out[0] = __uint_as_float(kX3Mark);
+            any_huge = 1;
+          }
         }
       }
     }
@@ -324,6 +343,20 @@ __global__ void __launch_bounds__(kX3Threads, W <= 64 ? 2 : 1) mlp_x3_kernel(con
   __syncthreads();
   tc_fence_after();
   if (warp == 0) tmem_dealloc(tmem, kCols);
+  // The marked rows last, when no other warp waits with a limit: a deep
+  // network's takes 0.1 ms.  The operands' memory is free by now.
+  if (any_huge == 0) return;
+  float* h = reinterpret_cast<float*>(smem) + warp * 256;
+  for (int64_t j = warp;; j += kX3Threads / 32) {  // 32 rows of the block's tiles each
+    const int64_t q0 = (blockIdx.x + j / 4 * gridDim.x) * kTcRows + j % 4 * 32;
+    if (q0 >= p.n) break;
+    unsigned marked = __ballot_sync(0xffffffffu, q0 + lane < p.n &&
+                                                     __float_as_uint(p.out[(q0 + lane) * p.out_stride]) == kX3Mark);
+    for (; marked; marked &= marked - 1) {
+      const int64_t q = q0 + __ffs(marked) - 1;
+      x3_plain_row(p.d, p.params, p.X + q * p.in_pad, h, p.out + q * p.out_stride, p.out_ch);
+    }
+  }
 }
 
 // The planes of every matrix (adam_kernel keeps them up to date afterwards).
