@@ -11,6 +11,7 @@
 #include <string>
 #include <vector>
 
+#include "hm_branch.h"
 #include "hm_hair_grad.cuh"
 #include "hm_mlp.cuh"
 #include "hm_render.h"
@@ -862,6 +863,8 @@ static int render_frame(Render* r, cudaStream_t user, bool sync_bounces) {
   // Instrumented frames run the stages one after another on one stream.
   const cudaStream_t sh = sync_bounces ? st : sl.st_shadow;
   auto trace = [&](const FrameParams& tfp) -> int {
+    SideBranch shadow(st, sh, sl.ev_shaded, sl.ev_resolved);
+    auto branch = [](cudaError_t e) { return e == cudaSuccess ? HM_OK : hm_cuda_status(e, "shadow branch"); };
     int* q_cur = sl.q_a;
     int* q_next = sl.q_b;
     int* c_cur = sl.counts;
@@ -884,7 +887,7 @@ static int render_frame(Render* r, cudaStream_t user, bool sync_bounces) {
                                                        sl.fetch + 2 * it, sl.err, r->d_cnt, counting,
                                                        r->blocks_extend, st))
         return e;
-      if (sh != st && it > 0) cudaStreamWaitEvent(st, sl.ev_resolved, 0);
+      if (int e = branch(shadow.join())) return e;
       mark(S_SHADE);
       if (tfp.mode == MODE_NRC) {
         if (int e = launch_nrc_shade(sd, tfp, sl.ps, fb_trace, sl.nrc, q_cur, c_cur, {sl.keep, s_cur}, grid, st)) return e;
@@ -892,10 +895,7 @@ static int render_frame(Render* r, cudaStream_t user, bool sync_bounces) {
         if (int e = launch_shade(sd, tfp, r->batch, sl.ps, fb_trace, q_cur, c_cur, {sl.keep, s_cur}, grid, st)) return e;
       }
       mark(S_SHADOW);
-      if (sh != st) {
-        cudaEventRecord(sl.ev_shaded, st);
-        cudaStreamWaitEvent(sh, sl.ev_shaded, 0);
-      }
+      if (int e = branch(shadow.fork())) return e;
       if (int e = launch_persistent<ShadowRays, true>(ShadowRays{sl.ps, q_cur, c_cur, sl.vis}, sd, r->batch, 0.f,
                                                       1e30f, sl.fetch + 2 * it + 1, sl.err, r->d_cnt + 3, counting,
                                                       r->blocks_shadow, sh))
@@ -904,7 +904,7 @@ static int render_frame(Render* r, cudaStream_t user, bool sync_bounces) {
                                                          tfp.mode == MODE_NRC ? sl.nrc.dl_rec : nullptr,
                                                          sl.nrc.rec, tfp.log);
       HM_CHECK_LAUNCH("shadow_resolve_kernel");
-      if (sh != st) cudaEventRecord(sl.ev_resolved, sh);
+      if (int e = branch(shadow.end())) return e;
       mark(S_COMPACT);
       compact_kernel<<<std::min(nblocks, r->sm_count * 2), kScanBlock, 0, st>>>(sl.keep, q_cur, c_cur, s_cur, q_next,
                                                                                 c_next, s_next, nblocks);
@@ -921,8 +921,7 @@ static int render_frame(Render* r, cudaStream_t user, bool sync_bounces) {
       std::swap(s_cur, s_next);
       ++bounces;
     }
-    if (sh != st && bounces > 0) cudaStreamWaitEvent(st, sl.ev_resolved, 0);
-    return HM_OK;
+    return branch(shadow.join());
   };
   if (r->graphs && !sync_bounces) {
     // the same launches as a graph per slot, captured once and replayed;
