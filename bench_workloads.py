@@ -990,7 +990,7 @@ class DiffBenchWorkload:
 
     @property
     def kernels_per_step(self):
-        # forward frames (bounce loop, cache inference, compose) + replay frames
+        # forward frames (frame number, bounce loop, cache inference, compose) + replay frames
         # (bounce loop, cache adjoint, two gradient sums) + group duals, total,
         # cache forward + backward
         rounds = 3  # BETA + 1 vertices at BETA = 2
@@ -998,7 +998,7 @@ class DiffBenchWorkload:
         # weight-gradient partials and their sum, hash-grid scatter and
         # conversion)
         mlp = 2 + 3 + 2
-        fwd = 1 + 5 * rounds + 1 + 2 + 1
+        fwd = 1 + 1 + 5 * rounds + 1 + 2 + 1
         rep = 1 + 5 * rounds + 3
         return self.spp * (fwd + rep) + 2 + mlp
 

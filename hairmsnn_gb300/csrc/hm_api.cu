@@ -13,6 +13,8 @@ void hm_set_error(const char* fmt, ...) {
   va_end(ap);
 }
 
+thread_local int64_t hm_launches = 0;
+
 int hm_cuda_status(cudaError_t e, const char* what) {
   cudaGetLastError();  // reported here: the next launch's check must not find it again
   hm_set_error("%s: %s (%s)", what, cudaGetErrorName(e), cudaGetErrorString(e));

@@ -83,8 +83,11 @@ HM_HD float lcg_next(uint32_t& s) {
 // Error plumbing for the C ABI (thread-local message, hm_last_error()).
 void hm_set_error(const char* fmt, ...);
 int hm_cuda_status(cudaError_t e, const char* what);
+// Kernel launches of this thread so far, counted by their check.
+extern thread_local int64_t hm_launches;
 #define HM_CHECK_LAUNCH(what)                                   \
   do {                                                          \
     cudaError_t _e = cudaGetLastError();                        \
     if (_e != cudaSuccess) return hm_cuda_status(_e, what);     \
+    ++hm_launches;                                              \
   } while (0)

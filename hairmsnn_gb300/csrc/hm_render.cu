@@ -457,6 +457,7 @@ struct Slot {
   // replayed every frame of this slot; the frame number comes from d_frame
   int* d_frame = nullptr;
   cudaGraphExec_t trace_exec = nullptr;
+  int64_t trace_launches = 0;  // kernels in it
   int64_t trace_key[10] = {};
   NrcBufs nrc{};  // NRC renderers
   // path replay (allocated by the first differentiable forward)
@@ -812,6 +813,7 @@ static int render_frame(Render* r, cudaStream_t user, bool sync_bounces) {
   SceneDev sd = s->dev();
   Slot& sl = r->slots[r->accum_id % r->depth];
   if (int e = slot_finish(r, sl)) return e;  // back-pressure: the slot's previous frame
+  int64_t launches = -hm_launches;  // the frame's: what is launched from here on
   const cudaStream_t st = sl.st;
   cudaEventRecord(r->ev_submit, user);
   cudaStreamWaitEvent(st, r->ev_submit, 0);
@@ -939,7 +941,10 @@ static int render_frame(Render* r, cudaStream_t user, bool sync_bounces) {
       cudaGraph_t g = nullptr;
       cudaError_t e = cudaStreamBeginCapture(st, cudaStreamCaptureModeRelaxed);
       if (e != cudaSuccess) return hm_cuda_status(e, "trace graph capture");
+      sl.trace_launches = -hm_launches;
       const int te = trace(tfp);
+      sl.trace_launches += hm_launches;
+      launches -= sl.trace_launches;  // recorded, not launched
       e = cudaStreamEndCapture(st, &g);
       if (te != HM_OK || e != cudaSuccess) {
         if (g) cudaGraphDestroy(g);
@@ -952,6 +957,7 @@ static int render_frame(Render* r, cudaStream_t user, bool sync_bounces) {
     }
     cudaError_t e = cudaGraphLaunch(sl.trace_exec, st);
     if (e != cudaSuccess) return hm_cuda_status(e, "trace graph launch");
+    launches += sl.trace_launches;
     bounces = rounds;
   } else {
     if (int e = trace(fp)) return e;
@@ -959,7 +965,6 @@ static int render_frame(Render* r, cudaStream_t user, bool sync_bounces) {
   r->rays_extend += ext_rays;
   r->last_bounces = bounces;
   cur_bounce = -1;
-  int launches = 1 + 5 * bounces + 1;
   if (r->mode == MODE_NRC) {
     // G_BUFFER done; then inference, RENDER pass (compose + training data),
     // training step (render_nrc.cu:651-681)
@@ -981,10 +986,6 @@ static int render_frame(Render* r, cudaStream_t user, bool sync_bounces) {
     }
     cudaEventRecord(r->ev_mlp, st);
     r->have_mlp_ev = true;
-    hm_mlp_desc md;
-    hm_mlp_info(r->mlp, &md);
-    const bool grid_enc = md.n_params > md.n_network_params;
-    launches += (r->train ? 5 + (grid_enc ? 2 : 0) : 0) + 2 + 2;
   } else if (r->mode == MODE_PT) {
     // writePixel accumulates: frames in order, after any pending read-back
     if (r->have_compose_ev) cudaStreamWaitEvent(st, r->ev_compose, 0);
@@ -1013,10 +1014,6 @@ static int render_frame(Render* r, cudaStream_t user, bool sync_bounces) {
     if (int e = launch_compose(r->P, fp, fb, st)) return e;
     cudaEventRecord(r->ev_compose, st);
     r->have_compose_ev = true;
-    hm_mlp_desc md;
-    hm_mlp_info(r->mlp, &md);
-    const bool grid_enc = md.n_params > md.n_network_params;
-    launches += (r->train && !r->diff_fwd ? 5 + (grid_enc ? 2 : 0) : 0) + 2 + 1;
   }
   mark(S_END);
   cudaMemcpyAsync(sl.h_err, sl.err, sizeof(int), cudaMemcpyDeviceToHost, st);
@@ -1027,7 +1024,7 @@ static int render_frame(Render* r, cudaStream_t user, bool sync_bounces) {
   memset(&tm, 0, sizeof(tm));
   tm.bounces = bounces;
   tm.extension_rays = ext_rays;
-  tm.kernel_launches = launches;
+  tm.kernel_launches = (int)(launches + hm_launches);
   if (r->timing && sync_bounces) {
     cudaEventSynchronize(r->event(ne - 1));
     float* slot[] = {&tm.camera_ms, &tm.extend_ms, &tm.shade_ms, &tm.shadow_ms, &tm.compact_ms,
