@@ -769,6 +769,7 @@ struct Mlp {
   float* Xi = nullptr;       // [xi_cap][in_pad] encoded inputs of an inference
   float* loss_dev = nullptr;
   long long* grid_acc = nullptr;  // fixed-point hash-grid gradient accumulator
+  bool grid_clear = false;        // grid_acc is zero once the work enqueued so far has run
   int64_t last_n = 0;        // batch of the last forward(), 0 while its buffers hold none
   const float* last_in = nullptr;
   // The weights as the tensor-core kernels read them (FP32 handles: three
@@ -902,11 +903,18 @@ static int encode(Mlp* m, const float* in, float* X, int64_t n, cudaStream_t st)
 // Hash-grid gradients of the last forward's batch from the input gradients dX.
 static int grid_backward(Mlp* m, const float* dX, int64_t n, cudaStream_t st) {
   const MlpDims& d = m->cfg.d;
-  if (!m->grid_acc) {  // cleared once here, then by every conversion
-    cudaError_t e = cudaMalloc(&m->grid_acc, d.n_enc_params * sizeof(long long));
-    if (e == cudaSuccess) e = cudaMemsetAsync(m->grid_acc, 0, d.n_enc_params * sizeof(long long), st);
-    if (e != cudaSuccess) return hm_cuda_status(e, "grid grad accumulator");
-  }
+  // The conversion clears the accumulator for the next batch.  It is cleared
+  // first where that is not known to have run: the first time, after a call
+  // that failed between the two, and in a graph, whose conversion runs when it
+  // is replayed, if it is.
+  const size_t bytes = d.n_enc_params * sizeof(long long);
+  cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+  cudaError_t e = cudaStreamIsCapturing(st, &capture);
+  if (e == cudaSuccess && !m->grid_acc) e = cudaMalloc(&m->grid_acc, bytes);
+  const bool captured = capture != cudaStreamCaptureStatusNone;
+  if (e == cudaSuccess && (captured || !m->grid_clear)) e = cudaMemsetAsync(m->grid_acc, 0, bytes, st);
+  if (e != cudaSuccess) return hm_cuda_status(e, "grid grad accumulator");
+  m->grid_clear = false;
   for (int si = 0; si < d.n_segs; ++si) {
     const EncSeg& s = d.segs[si];
     if (s.type != ENC_HASHGRID) continue;
@@ -916,6 +924,7 @@ static int grid_backward(Mlp* m, const float* dX, int64_t n, cudaStream_t st) {
   }
   grid_fix_to_float_kernel<<<1024, 256, 0, st>>>(m->grid_acc, m->grads + d.n_net_params, d.n_enc_params);
   HM_CHECK_LAUNCH("grid_fix_to_float_kernel");
+  m->grid_clear = !captured;
   return HM_OK;
 }
 
