@@ -993,12 +993,16 @@ extern "C" hm_mlp* hm_mlp_create(const char* config_json, int in_ch, int out_ch,
   m->precision = precision;
   m->n_params = m->cfg.d.n_net_params + m->cfg.d.n_enc_params;
   m->lr = m->cfg.adam.lr;
+  m->tc_train = precision != HM_PREC_FP32 && tc_trainable(m->cfg.d, precision);
+  // FP16 operands in the backward pass (FP16 handles; E4M3 handles' backward)
+  m->loss_scale = precision == HM_PREC_FP16 || precision == HM_PREC_FP8_E4M3 ? 128.f : 1.f;
   size_t bytes = m->n_params * sizeof(float);
   cudaError_t e = cudaMalloc(&m->params, bytes);
   if (e == cudaSuccess) e = cudaMalloc(&m->grads, bytes);
   if (e == cudaSuccess) e = cudaMalloc(&m->adam_m, bytes);
   if (e == cudaSuccess) e = cudaMalloc(&m->adam_v, bytes);
   if (e == cudaSuccess) e = cudaMalloc(&m->loss_dev, sizeof(float));
+  if (e == cudaSuccess && m->loss_scale != 1.f) e = cudaMalloc(&m->grads_out, bytes);
   if (e == cudaSuccess) e = cudaHostAlloc(&m->tc_err_host, sizeof(int), cudaHostAllocMapped);
   if (e == cudaSuccess) {
     *m->tc_err_host = 0;
@@ -1008,9 +1012,6 @@ extern "C" hm_mlp* hm_mlp_create(const char* config_json, int in_ch, int out_ch,
   if (e == cudaSuccess && precision != HM_PREC_FP32) {
     int st = tc_pack_alloc(m->cfg.d, precision, &m->tc);
     if (st != HM_OK) e = cudaErrorMemoryAllocation;
-    m->tc_train = tc_trainable(m->cfg.d, precision);
-    // FP16 operands in the backward pass (FP16 handles; E4M3 handles' backward)
-    m->loss_scale = precision == HM_PREC_FP16 || precision == HM_PREC_FP8_E4M3 ? 128.f : 1.f;
   }
   if (e != cudaSuccess) {
     *status = hm_cuda_status(e, "hm_mlp_create");
@@ -1086,19 +1087,16 @@ extern "C" int hm_mlp_set_params(hm_mlp* h, const float* host_in) {
 }
 
 extern "C" int hm_mlp_get_gradients(const hm_mlp* h, float* host_out) {
-  Mlp* m = const_cast<Mlp*>((const Mlp*)h);  // grads_out is a lazily made buffer
+  const Mlp* m = (const Mlp*)h;
   if (!m || !host_out) return hm_set_error("hm_mlp_get_gradients: NULL"), HM_EINVAL;
   const float* src = m->grads;
   cudaError_t e = cudaSuccess;
   if (m->tc_train && m->loss_scale != 1.f) {
     // undo the FP16 loss scale (a power of two: exact) on the device: over the
     // renderer's million gradients the host loop took 0.2 ms of a 0.43 ms step
-    if (!m->grads_out) e = cudaMalloc(&m->grads_out, m->n_params * sizeof(float));
-    if (e == cudaSuccess) {
-      unscale_kernel<<<1024, 256>>>(m->grads, 1.f / m->loss_scale, m->grads_out, m->n_params);
-      e = cudaGetLastError();
-      src = m->grads_out;
-    }
+    unscale_kernel<<<1024, 256>>>(m->grads, 1.f / m->loss_scale, m->grads_out, m->n_params);
+    e = cudaGetLastError();
+    src = m->grads_out;
   }
   if (e == cudaSuccess) e = cudaMemcpy(host_out, src, m->n_params * sizeof(float), cudaMemcpyDeviceToHost);
   return e == cudaSuccess ? HM_OK : hm_cuda_status(e, "hm_mlp_get_gradients");
