@@ -750,6 +750,12 @@ __global__ void __launch_bounds__(kTcThreads, 2) mlp_tc_fwd_kernel(const __grid_
 #pragma unroll
         for (int e = 0; e < 16; ++e) v[c * 16 + e] = fmaxf(F8 ? t[e] * sc : t[e], 0.f);
       }
+      if constexpr (HW == 8) {  // width 16: eight columns of one load each
+        float t[16];
+        tmem_ld16(row_taddr, t);
+#pragma unroll
+        for (int e = 0; e < 8; ++e) v[e] = fmaxf(half ? t[8 + e] : t[e], 0.f);
+      }
       if (F8) {
         float amax = 0.f;
 #pragma unroll
@@ -1596,6 +1602,22 @@ __global__ void __launch_bounds__(kTcThreads, 1) mlp_tc_bwd_kernel(const __grid_
       } else {
         constexpr int HW = W / 2;
         const uint16_t* hrow = p.h16 + ((int64_t)(j - 1) * p.n + (valid ? q : 0)) * W + half * HW;
+        if constexpr (HW == 8) {  // width 16: eight columns of one load each
+          float t[16];
+          tmem_ld16(row_taddr, t);
+          const uint4 hv = valid ? __ldg(reinterpret_cast<const uint4*>(hrow)) : make_uint4(0, 0, 0, 0);
+          const uint16_t* hs = reinterpret_cast<const uint16_t*>(&hv);
+          float g[8];
+#pragma unroll
+          for (int e = 0; e < 8; ++e) {
+            const float te = half ? t[8 + e] : t[e];
+            g[e] = hs[e] != 0 && !(hs[e] & 0x8000) ? te : 0.f;
+          }
+          const uint4 word = make_uint4(pack2<PREC>(g[0], g[1]), pack2<PREC>(g[2], g[3]), pack2<PREC>(g[4], g[5]),
+                                        pack2<PREC>(g[6], g[7]));
+          *reinterpret_cast<uint4*>(A + op_offset(kTcRows, row, half * 16)) = word;
+          if (valid) *reinterpret_cast<uint4*>(p.dz16 + ((int64_t)(j - 1) * p.n + q) * p.wz + half * 8) = word;
+        }
 #pragma unroll
         for (int c = 0; c < HW / 16; ++c) {
           float t[16];
