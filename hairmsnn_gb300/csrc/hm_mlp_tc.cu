@@ -1495,6 +1495,8 @@ struct TcBwdArgs {
   int wz;  // row pitch of dz16 (max(W, 16))
 };
 
+constexpr int kTcMaxN = 256;  // columns of one MMA
+
 template <int PREC, int W>
 __global__ void __launch_bounds__(kTcThreads, 1) mlp_tc_bwd_kernel(const __grid_constant__ TcBwdArgs p) {
   constexpr int FMT = PREC == TC_BF16 ? 1 : 0;
@@ -1529,12 +1531,13 @@ __global__ void __launch_bounds__(kTcThreads, 1) mlp_tc_bwd_kernel(const __grid_
   bool failed = false;
   float loss_acc = 0.f;
 
-  auto run = [&](int j, int k_count) -> bool {  // MMAs of dH_j = dZ_{j+1} W_j
+  // MMAs of columns [n0, n0 + n_count) of dH_j = dZ_{j+1} W_j
+  auto run = [&](int j, int k_count, int n0, int n_count) -> bool {
     if (tid == 0) {
       tc_fence_after();
-      const uint32_t idesc = tc_idesc(kTcRows, p.NT[j], FMT);
+      const uint32_t idesc = tc_idesc(kTcRows, n_count, FMT);
       const uint32_t b_lbo = 16 * p.NT[j];
-      const uint32_t b_base = w_base + (uint32_t)p.boff_t[j];
+      const uint32_t b_base = w_base + (uint32_t)p.boff_t[j] + (uint32_t)op_offset(p.NT[j], n0, 0);
       for (int ks = 0; ks < k_count / 16; ++ks) {
         const uint64_t ad = tc_sdesc(a_base + (uint32_t)ks * 2 * a_lbo, a_lbo, 128);
         const uint64_t bd = tc_sdesc(b_base + (uint32_t)ks * 2 * b_lbo, b_lbo, 128);
@@ -1585,21 +1588,30 @@ __global__ void __launch_bounds__(kTcThreads, 1) mlp_tc_bwd_kernel(const __grid_
     __syncthreads();
     int kk = 16;  // K of the next MMA: columns of the dZ in A
     for (int j = L; j >= 0 && !failed; --j) {
-      if (j == 0 && !p.dX) break;
-      if (!run(j, kk)) {
-        failed = true;
-        break;
-      }
-      const int nt = p.NT[j];  // inputs of layer j: W (j >= 1) or K0 (j == 0)
       if (j == 0) {
-        // dX (loss-scaled, FP32) for the hash-grid backward
-        for (int c = half * 16; c < nt; c += 32) {
-          float t[16];
-          tmem_ld16(row_taddr + c, t);
-          if (valid)
-            for (int e = 0; e < 16 && c + e < d.in_pad; ++e) p.dX[q * d.in_pad + c + e] = t[e];
+        // dX (loss-scaled, FP32) for the hash-grid backward, 256 columns (the
+        // widest MMA) at a time
+        if (!p.dX) break;
+        for (int n0 = 0; n0 < p.NT[0] && !failed; n0 += kTcMaxN) {
+          const int nt = min(kTcMaxN, p.NT[0] - n0);
+          if (!run(0, kk, n0, nt)) {
+            failed = true;
+            break;
+          }
+          for (int c = half * 16; c < nt; c += 32) {
+            float t[16];
+            tmem_ld16(row_taddr + c, t);
+            if (valid)
+              for (int e = 0; e < 16 && n0 + c + e < d.in_pad; ++e) p.dX[q * d.in_pad + n0 + c + e] = t[e];
+          }
+          tc_fence_before();
+          __syncthreads();
         }
       } else {
+        if (!run(j, kk, 0, W)) {
+          failed = true;
+          break;
+        }
         constexpr int HW = W / 2;
         const uint16_t* hrow = p.h16 + ((int64_t)(j - 1) * p.n + (valid ? q : 0)) * W + half * HW;
         if constexpr (HW == 8) {  // width 16: eight columns of one load each
@@ -1903,7 +1915,7 @@ int tc_backward(const MlpDims& d, const TcPack& pk, const TcTrainBufs& b, const 
   a.err = err_flag;
   a.wz = std::max(W, 16);
   int ncols = 32;
-  while (ncols < std::max(W, need_dx ? pk.NT[0] : 16)) ncols *= 2;
+  while (ncols < std::max(W, need_dx ? std::min(pk.NT[0], kTcMaxN) : 16)) ncols *= 2;
   a.ncols = ncols;
   a.a_bytes = kTcRows * std::max(W, 16) * 2;
   const size_t smem = (size_t)a.a_bytes + ((pk.bytes_t + 127) & ~(int64_t)127) + 64 + 1024 + 64;
