@@ -29,6 +29,7 @@ struct HairConsts {
   float mp_den[3];    // sinh(1 / v[k]) * 2 * v[k]
   float exp_m2v[4];   // exp(-2 / v[p]), p = 0..3
   int fp64_mp;        // beta_m < 0.1
+  double mp_inv_d[3], mp_logc_d[3];  // then: 1 / v[k] and log(1 / (2 v[k])) in FP64
 };
 
 HM_HD float logistic_cdf_s(float x, float s) { return 1.f / (1.f + expf(-x / s)); }  // LogisticCDF :123-125
@@ -65,6 +66,10 @@ HM_HD HairConsts hair_consts(const hm_hair_params& p) {
   }
   for (int k = 0; k < 4; ++k) hc.exp_m2v[k] = expf(-2.f / hc.v[k]);
   hc.fp64_mp = bm < 0.1f ? 1 : 0;
+  for (int k = 0; k < 3; ++k) {
+    hc.mp_inv_d[k] = hc.fp64_mp ? 1.0 / (double)hc.v[k] : 0.0;
+    hc.mp_logc_d[k] = hc.fp64_mp ? log(1.0 / (2.0 * (double)hc.v[k])) : 0.0;
+  }
   return hc;
 }
 
@@ -127,20 +132,24 @@ HM_D double bessel_i0_d(double x) {
 // into every lobe of every evaluation its logarithms and exponential made the
 // kernels larger than the instruction caches: five to eight issue slots lost
 // to fetching for each instruction of the shading kernel, and bsdf_eval_kernel
-// took 36 us for 262,144 queries instead of 22.
-static __device__ __noinline__ float mp_lobe_fp64(float cti, float cto, float sti, float sto, float v) {
+// took 36 us for 262,144 queries instead of 22.  Where it runs it is bound by
+// the FP64 units; the material's two terms come with the constants (2,000,003
+// queries at beta_m 0.09: 3203 us inlined with those terms in every lobe, 3324
+// called, 2721 now).
+static __device__ __noinline__ float mp_lobe_fp64(float cti, float cto, float sti, float sto, float v, double inv_v,
+                                                  double logc) {
   double dv = v;
   double a = (double)cti * (double)cto / dv;
   double b = (double)sti * (double)sto / dv;
   double li = a > 12.0 ? a + 0.5 * (-log(2.0 * (double)kPi) + log(1.0 / a) + 1.0 / (8.0 * a))
                        : log(bessel_i0_d(a));
-  return (float)exp(li - b - 1.0 / dv + 0.6931 + log(1.0 / (2.0 * dv)));
+  return (float)exp(li - b - inv_v + 0.6931 + logc);
 }
 
 // M_p (disney_hair.cuh:78-88) for lobe constants k; v = v[k].
 HM_D float mp_lobe(float cti, float cto, float sti, float sto, const HairConsts& hc, int k) {
   const float v = hc.v[k];
-  if (hc.fp64_mp && v <= 0.1f) return mp_lobe_fp64(cti, cto, sti, sto, v);
+  if (hc.fp64_mp && v <= 0.1f) return mp_lobe_fp64(cti, cto, sti, sto, v, hc.mp_inv_d[k], hc.mp_logc_d[k]);
   float a = cti * cto / v;
   float b = sti * sto / v;
   if (v <= 0.1f) return expf(log_i0(a) - b - hc.inv_v[k] + 0.6931f + hc.mp_logc[k]);
