@@ -19,11 +19,12 @@ HairConsts hair_consts_from_params(const hm_hair_params& p) { return hair_consts
 
 HM_D float ldg(const float* p) { return __ldg(p); }
 
-// Bound by instruction issue (about 1,500 and 1,900 instructions per query;
-// 75% of the issue slots used, 14% of HBM).  Six 256-thread blocks per SM (40
-// registers, a few spills to L1).  8,000,003 queries: eval 366 us, sample 463
-// at six blocks, 369 / 456 at four (before the lobe loop, the exact constant
-// divisions and the geometry shared by sample and evaluation: 493 / 700 us).
+// Bound by instruction issue (1,600 and 1,950 warp instructions per 32 queries,
+// 88% and 85% of the issue slots used, HBM at 17% and 19%).  Six 256-thread
+// blocks per SM (40 registers, a few spills to L1).  8,000,003 queries: eval
+// 372 us, sample 470 at six blocks; 1.01 and 0.98 times that at four.  Before
+// the lobe loop, the exact constant divisions and the geometry shared by sample
+// and evaluation: 493 / 700 us.
 __global__ void __launch_bounds__(256, 6) bsdf_eval_kernel(HairConsts hc, const float* __restrict__ wo,
                                                         const float* __restrict__ wi,
                                                         const float* __restrict__ t,
@@ -157,13 +158,10 @@ extern "C" int hm_bsdf_eval(const hm_bsdf_queries* q, float* f, float* pdf, int6
 // registers and the material's terms made by every thread.
 constexpr int kGradThreads = 128;
 constexpr int kGradPerSm = 6;  // blocks per SM
-__global__ void __launch_bounds__(kGradThreads, kGradPerSm) bsdf_eval_grad_kernel(hm_hair_params p, const float* __restrict__ wo,
-                                                             const float* __restrict__ wi,
-                                                             const float* __restrict__ t,
-                                                             const float* __restrict__ h,
-                                                             float* __restrict__ f, float* __restrict__ pdf,
-                                                             float* __restrict__ df, float* __restrict__ dpdf,
-                                                             int64_t n) {
+__global__ void __launch_bounds__(kGradThreads, kGradPerSm)
+    bsdf_eval_grad_kernel(hm_hair_params p, const float* __restrict__ wo, const float* __restrict__ wi,
+                          const float* __restrict__ t, const float* __restrict__ h, float* __restrict__ f,
+                          float* __restrict__ pdf, float* __restrict__ df, float* __restrict__ dpdf, int64_t n) {
   const float gain[4] = {p.gain_r, p.gain_tt, p.gain_trt, p.gain_trrt};
   __shared__ HairConstsD hc;
   if (threadIdx.x == 0) hc = hair_consts_dual(p.sigma_a, p.beta_m, p.beta_n, p.alpha, gain);
@@ -192,8 +190,8 @@ extern "C" int hm_bsdf_eval_grad(const hm_bsdf_queries* q, float* f, float* pdf,
   if (n == 0) return HM_OK;
   if (!q->wo || !q->wi || !q->tangent || !q->h || !f || !pdf || !df)
     return hm_set_error("hm_bsdf_eval_grad: NULL array"), HM_EINVAL;
-  bsdf_eval_grad_kernel<<<grid_for(n, kGradThreads, kGradPerSm), kGradThreads, 0, (cudaStream_t)stream>>>(*params, q->wo, q->wi, q->tangent, q->h,
-                                                                             f, pdf, df, dpdf, n);
+  bsdf_eval_grad_kernel<<<grid_for(n, kGradThreads, kGradPerSm), kGradThreads, 0, (cudaStream_t)stream>>>(
+      *params, q->wo, q->wi, q->tangent, q->h, f, pdf, df, dpdf, n);
   HM_CHECK_LAUNCH("bsdf_eval_grad_kernel");
   return HM_OK;
 }

@@ -78,10 +78,9 @@ HairConsts hair_consts_from_params(const hm_hair_params& p);
 
 // a / c for a positive constant c whose reciprocal is a compile-time constant:
 // the quotient estimate, its exact remainder and one correction (Markstein,
-// IBM J. Res. Dev. 34, 1990), three instructions instead of a division's ten.
-// For every c used here this is the correctly rounded quotient of every
-// normal a (checked over all mantissas, tests/test_div_const.py), so results
-// keep their bits; a must not be infinite.
+// IBM J. Res. Dev. 34, 1990).  For every c used here this is the correctly rounded quotient of every
+// normal a (checked over all mantissas, tests/test_div_const_header.py), so
+// results keep their bits; a must not be infinite.
 HM_HD float div_const(float a, float c) {
   const float y = 1.f / c;
 #ifdef __CUDA_ARCH__
@@ -234,9 +233,9 @@ HM_D HairEval hair_eval(const HairGeom& g, f3 wi, const HairConsts& hc) {
   // M_p and N_p of the lobes R, TT, TRT, TRRT.  R tilts by -2^1 alpha, TT by
   // 2^0, TRT by 2^2, TRRT not (the sine's sign carries the direction exactly).
   // A loop, not unrolled: the four copies of a lobe's code overran the
-  // instruction caches.  bsdf_sample_kernel, 8,000,003 queries: 672 us
-  // unrolled, 632 as a loop; its sums f and pdf stay outside the loop (713
-  // inside it, with the values they keep alive).
+  // instruction caches.  bsdf_sample_kernel, 8,000,003 queries: 502 us unrolled,
+  // 470 as a loop; its sums f and pdf stay outside the loop (494 inside it,
+  // with the values they keep alive).
   float mp[4], np[3];
 #pragma unroll 1
   for (int p = 0; p < 4; ++p) {

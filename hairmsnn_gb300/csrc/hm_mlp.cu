@@ -181,12 +181,13 @@ MlpConfig mlp_config_from_json(const char* text, int in_ch, int out_ch) {
 // divergence and a level's eight corner gathers are in flight together.  The
 // rows are collected in shared memory (row pitch odd: a column of 32 rows
 // falls into 32 banks) and written to X in whole lines.
-// Bound by the corner gathers' latency and L2 sectors (hash grids) or by the
-// sines and edges (Frequency / OneBlob).  One thread per query, writing its
-// own row, took 278 us for 262,144 queries of the hash-grid network and
-// 113 us for 517 of them (128 dependent gathers one after another); now 97 and
-// 7 us (whole calls at four / five / six blocks per SM: 162 / 156 / 177 us).  Loading the two corners
-// of an aligned pair of entries as one 16 bytes changed nothing.
+// Bound by the corner gathers (hash grids: L1 81%, L2 60% busy) or by the issue
+// of the sines and edges (Frequency / OneBlob: 86% of the slots).  One thread
+// per query, writing its own row, took 278 us for 262,144 queries of the
+// hash-grid network and 113 us for 517 of them (128 dependent gathers one after
+// another); now 99 and 7 us (whole calls at four / five / six blocks per SM:
+// 162 / 156 / 177 us).  Loading the two corners of an aligned pair of entries
+// as one 16 bytes changed nothing.
 constexpr int kEncRows = 32;
 constexpr int kEncThreads = 256;
 
@@ -466,12 +467,10 @@ __global__ void __launch_bounds__(256) mlp_fwd_kernel(const __grid_constant__ Ml
 #pragma unroll
       for (int j = 0; j < S::TO; ++j) Hout[(to * S::TO + j) * lda_in + tq * S::TQ + i] = fmaxf(acc[i][j], 0.f);
     __syncthreads();
-    if (acts) {  // store h_{l+1} as [n][W] row-major
-      float* dst = acts + (int64_t)l * n * W;
-      for (int i = threadIdx.x; i < BM * W; i += 256) {
-        int q = i / W, k = i % W;
-        if (q0 + q < n) dst[(q0 + q) * W + k] = Hout[k * lda_in + q];
-      }
+    float* dst = acts + (int64_t)l * n * W;  // h_{l+1} as [n][W] row-major
+    for (int i = threadIdx.x; i < BM * W; i += 256) {
+      int q = i / W, k = i % W;
+      if (q0 + q < n) dst[(q0 + q) * W + k] = Hout[k * lda_in + q];
     }
     A = Hout;
     K = W;
@@ -1562,9 +1561,10 @@ extern "C" int hm_mlp_describe_config(const char* config_json, int in_ch, int ou
 }
 
 // ============================================= inference without allocation
-// hm_mlp_inference_noalloc: the same kernels as hm_mlp_inference, but the encoded-input scratch ([n][in_pad] floats, the
-// only per-call device memory inference needs) lives in a fixed file-scope
-// device array instead of the handle's cudaMalloc'd workspace.  It exists for
+// hm_mlp_inference_noalloc: the same kernels as hm_mlp_inference, but the
+// encoded-input scratch ([n][in_pad] floats, the only device memory whose size
+// depends on the call) lives in a fixed file-scope device array instead of the
+// handle's cudaMalloc'd buffer.  It exists for
 // callers that may not allocate device memory once running: a frame loop that
 // reserves all of its memory up front and must not stall on cudaMalloc (which
 // can synchronise the device) or fail on it under memory pressure halfway
@@ -1575,7 +1575,7 @@ extern "C" int hm_mlp_describe_config(const char* config_json, int in_ch, int ou
 //    queries at in_pad 224, 16,384 at in_pad 64); larger n is rejected with
 //    HM_ECAPACITY and nothing is launched.  Split larger batches.
 //  * Nothing has to start at zero: the encode kernel writes every one of the
-//    first n * in_pad floats before the forward kernel reads them.
+//    first n * in_pad floats before the layers read them.
 //  * One scratch per device, shared by every handle: two calls whose work
 //    overlaps on the device (different streams, threads or handles without an
 //    ordering between them) overwrite each other's scratch.  Order them.

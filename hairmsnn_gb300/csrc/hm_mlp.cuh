@@ -179,8 +179,8 @@ int wgrad_sum(const WgradSum& r, const float* part, float* grads, const float* l
 // BF16 planes (x3_pack_bytes(d) bytes, written by what writes the parameters).
 int64_t x3_pack_bytes(const MlpDims& d);
 int x3_pack(const MlpDims& d, const float* params, uint8_t* blob, cudaStream_t st);
-int x3_forward(const MlpDims& d, const float* params, const uint8_t* blob, const float* X, float* out, int out_stride, int64_t n,
-               int* err_flag, cudaStream_t st);
+int x3_forward(const MlpDims& d, const float* params, const uint8_t* blob, const float* X, float* out, int out_stride,
+               int64_t n, int* err_flag, cudaStream_t st);
 
 // ---- tensor-core (tcgen05) forward for HM_PREC_FP16 / BF16 / FP8_E4M3
 // Weights are repacked from the FP32 master copy into the operand layout of

@@ -308,11 +308,10 @@ HM_D void enc_range(const MlpDims& d, const float* __restrict__ xin, const float
 // consecutive ones (circularly): its units are stored as zeros and the two or
 // three words that hold the five masses are stored over them, where the
 // mass-by-mass selection cost about eleven instructions per bin.
-// The kernels that encode are bound by instruction issue (31 per sincospif, 27
-// per OneBlob edge).  Feature by feature through the packing register of
-// enc_range -> by units: tc_encode_kernel<E4M3>, 300,007 queries of the 5 x 128
-// network 104 -> 41 us; mlp_tc_fused_kernel<FP16, 64>, 2^20 queries 498 -> 248
-// us (about 5000 instructions per query, 12,000 before).
+// The kernels that encode are bound by instruction issue.  Feature by feature
+// through the packing register of enc_range -> by units: tc_encode_kernel<E4M3>,
+// 300,007 queries of the 5 x 128 network 104 -> 41 us; mlp_tc_fused_kernel<FP16,
+// 64>, 2^20 queries 498 -> 240 us.
 //
 // The caller's row: operand bytes of feature k at
 //   a + (k * bytes / 16) * 2048 + k * bytes % 16    (128-row core-matrix layout)
@@ -1043,8 +1042,9 @@ struct TcPackArgs {
 // E4M3: amax of layer blockIdx.y's weights, blockIdx.y == n_layers: of the
 // encoding parameters (as integers: the bits of non-negative floats order as
 // the floats do, so the result does not depend on the blocks' order).
-__global__ void __launch_bounds__(256) tc_amax_kernel(const __grid_constant__ MlpDims d, const float* __restrict__ params,
-                                                      int n_layers, uint32_t* __restrict__ amax) {
+__global__ void __launch_bounds__(256) tc_amax_kernel(const __grid_constant__ MlpDims d,
+                                                      const float* __restrict__ params, int n_layers,
+                                                      uint32_t* __restrict__ amax) {
   __shared__ float red[8];
   const int l = blockIdx.y;
   int64_t begin, count;
@@ -1357,10 +1357,10 @@ int tc_forward(const MlpDims& d, const TcPack& pk, const float* enc_params, cons
   if (int e = tc_args(d, pk, enc_params, in, out, out_stride, n, err_flag, &a, &smem)) return e;
   const bool have_work = work && work_bytes >= tc_encode_bytes(d, pk, n);
   // The warp-specialised kernel wherever it fits, from the measured times
-  // (FP16, width 64; 517 / 65,536 / 2^20 queries): 17 / 26 / 247 us on the
-  // Frequency / OneBlob network and 17 / 35 / 340 us on the hash grid, against
-  // 23 / 33 / 305 and 17 / 36 / 401 us for the encode kernel + layer kernel
-  // and 17 / 30 / 333 and 17 / 60 / 662 us for the layer kernel encoding its
+  // (FP16, width 64; 517 / 65,536 / 2^20 queries): 16 / 26 / 240 us on the
+  // Frequency / OneBlob network and 17 / 35 / 347 us on the hash grid, against
+  // 23 / 34 / 308 and 18 / 38 / 404 us for the encode kernel + layer kernel
+  // and 18 / 32 / 335 and 18 / 61 / 666 us for the layer kernel encoding its
   // own tiles.
   const bool want_fz = g_tc_path != 1;
   if (want_fz) {
@@ -1694,9 +1694,10 @@ __global__ void __launch_bounds__(kTcThreads, 1) mlp_tc_bwd_kernel(const __grid_
 // transposes a K-major operand needs.  A feature group is padded by 16 bytes
 // so that the pieces of one row fall into different banks.
 // Bound by the serial chain over a chunk (32 stages of 64 rows); a ring of
-// four stages keeps three stages' copies in flight under the MMAs.  A whole
-// FP16 step on 65,536 rows of the 5 x 64 network: 319 us; with a launch and a
-// reduction per layer, 32 CTAs each and 2-byte transposing stores, 958 us.
+// four stages keeps three stages' copies in flight under the MMAs.  With a
+// launch and a reduction per layer, 32 CTAs each and 2-byte transposing stores
+// a FP16 step on 65,536 rows of the 5 x 64 network, gradients read back, took
+// 958 us, with this 319 (and 232 with the weights packed in one launch as well).
 constexpr int kWgRows = 64;                            // rows of a stage
 constexpr int kWgGroup = kWgRows / 8 * 128 + 16;       // bytes of one 8-feature group of a stage
 constexpr int kWgStages = 4;
@@ -1932,8 +1933,8 @@ int tc_backward(const MlpDims& d, const TcPack& pk, const TcTrainBufs& b, const 
   // weight gradients: jobs of one layer x a tile of its inputs.  64 inputs
   // per tile; 32 while that still gives at most one CTA per SM.  A whole
   // step, FP16, tiles of 256 / 128 / 64 / 32 inputs: 5 x 64 network, 65,536
-  // rows 339 / 333 / 319 / 354 us, 16,384 rows 240 / 226 / 219 / 213 us;
-  // 5 x 128, 16,384 rows 292 / 275 / 267 / 285 us.
+  // rows 207 / 206 / 189 / 223 us, 16,384 rows 125 / 113 / 101 / 96 us, 2,048
+  // rows 123 / 111 / 101 / 96 us; 5 x 128, 16,384 rows 160 / 144 / 134 / 152 us.
   int dev = 0, sms = 0;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);

@@ -2,14 +2,16 @@
 //
 // An FP32 value is the exact sum of three BF16 values (8 significand bits
 // each, FP32's exponent range): v = b0 + b1 + b2 with b0 = bf16(v), b1 =
-// bf16(v - b0), b2 = bf16(v - b0 - b1), each difference exact.  A layer's
-// product is formed from the six partial products whose weight is at least
-// 2^-16 of the first, in three FP32 accumulators:
+// bf16(v - b0), b2 = bf16(v - b0 - b1), each difference exact (the split of
+// Henry, Tang and Heinecke, ARITH 2019).  A layer's product is formed from the
+// six partial products whose weight is at least 2^-16 of the first, in three
+// FP32 accumulators:
 //   D0 = a0 w0,   D1 = a0 w1 + a1 w0,   D2 = a0 w2 + a1 w1 + a2 w0
-// and h = D0 + (D1 + D2).  What is left out is below 2^-25 of |a||w|.  The
-// tensor cores truncate when they accumulate, so D0 is kept as two sums, of
-// the even and of the odd 16-wide K steps: half the truncations in each.  With
-// the planes of W side by side as rows of one B operand, a K step is
+// and h = D0 + (D1 + D2).  What is left out, a1 w2 and a2 w1 above all, is below
+// 2^-24 of |a||w|.  The tensor cores truncate when they accumulate, so D0 is
+// kept as two sums, of the even and of the odd 16-wide K steps: half the
+// truncations in each.  With the planes of W side by side as rows of one B
+// operand, a K step is
 //   a0 x [w0 | w1 | w2] -> [D0 | D1 | D2]         (even steps)
 //   a0 x w0 -> D0', a0 x [w1 | w2] -> [D1 | D2]   (odd steps)
 //   a1 x [w0 | w1] -> [D1 | D2],  a2 x w0 -> D2.
@@ -32,10 +34,10 @@
 // expire too, and the block reports it and returns.
 //
 // Bound by the chain of a tile (A written, MMAs, accumulators read) with two
-// CTAs to fill it: issue slots and tensor pipe are each about a third busy.
-// The renderer's network, 262,144 queries: 246 us with FP32 multiply-adds ->
-// 63; whole calls, 200,003 queries: 5 x 64 network 1344 -> 245 us, 5 x 128
-// 3025 -> 411.
+// CTAs to fill it: 39% of the issue slots and 20% of the tensor pipe used.  The
+// renderer's network, 262,144 queries: 246 us with FP32 multiply-adds -> 64;
+// whole calls, 200,003 queries: 5 x 64 network 1344 -> 220 us, 5 x 128 3025 ->
+// 388.
 #include <cuda_bf16.h>
 
 #include <string.h>
@@ -388,8 +390,8 @@ static int x3_launch(const X3Args& a, size_t smem, cudaStream_t st) {
   return HM_OK;
 }
 
-int x3_forward(const MlpDims& d, const float* params, const uint8_t* blob, const float* X, float* out, int out_stride, int64_t n,
-               int* err_flag, cudaStream_t st) {
+int x3_forward(const MlpDims& d, const float* params, const uint8_t* blob, const float* X, float* out, int out_stride,
+               int64_t n, int* err_flag, cudaStream_t st) {
   X3Args a;
   memset(&a, 0, sizeof(a));
   a.d = d;

@@ -892,9 +892,11 @@ static int render_frame(Render* r, cudaStream_t user, bool sync_bounces) {
       if (int e = branch(shadow.join())) return e;
       mark(S_SHADE);
       if (tfp.mode == MODE_NRC) {
-        if (int e = launch_nrc_shade(sd, tfp, sl.ps, fb_trace, sl.nrc, q_cur, c_cur, {sl.keep, s_cur}, grid, st)) return e;
+        if (int e = launch_nrc_shade(sd, tfp, sl.ps, fb_trace, sl.nrc, q_cur, c_cur, {sl.keep, s_cur}, grid, st))
+          return e;
       } else {
-        if (int e = launch_shade(sd, tfp, r->batch, sl.ps, fb_trace, q_cur, c_cur, {sl.keep, s_cur}, grid, st)) return e;
+        if (int e = launch_shade(sd, tfp, r->batch, sl.ps, fb_trace, q_cur, c_cur, {sl.keep, s_cur}, grid, st))
+          return e;
       }
       mark(S_SHADOW);
       if (int e = branch(shadow.fork())) return e;

@@ -37,7 +37,6 @@ struct NrcBufs {
   int all_unbiased;
 };
 
-// Structure-of-arrays path state, one slot per pixel (capacity W*H).
 // What a shading launch leaves for the queue's compaction: flag[i] = 1 if path
 // queue[i] continues, sums[i / kScanBlock] += 1 for it (sums is zero before).
 constexpr int kScanBlock = 1024;
@@ -46,6 +45,7 @@ struct KeepOut {
   int* __restrict__ sums;
 };
 
+// Structure-of-arrays path state, one slot per pixel (capacity W*H).
 struct PathState {
   uint32_t* rng;
   uint32_t* flags;

@@ -747,7 +747,6 @@ SceneDev Scene::dev() const {
   d.alpha = a * a;
   d.nodes = d_nodes;
   d.n_nodes = n_nodes;
-  d.prim_of_leaf = d_prim_of_leaf;
   d.leaf_info = d_leaf_info;
   d.wnodes = d_wnodes;
   d.n_wnodes = n_wnodes;

@@ -45,7 +45,6 @@ struct SceneDev {
   // BVH over [segments | triangles]: node i has two children (child AABBs inline)
   const float4* nodes;  // 4 float4 per node
   int n_nodes;
-  const int* prim_of_leaf;  // leaf slot -> primitive id
   const int2* leaf_info;    // leaf slot -> (first control point of its segment, or ~triangle; primitive id)
   // the same tree collapsed to kWide-wide nodes (what the traversal walks):
   // kWideF4 float4 per node, lo.x[8] hi.x[8] lo.y[8] hi.y[8] lo.z[8] hi.z[8]
