@@ -119,6 +119,7 @@ constexpr int kParkAnyHit = 2;        // leaves a lane parks before the leaf pha
 constexpr int kParkClosest = 2;       // ... extension rays
 constexpr bool kAnyHitNearest = false;  // shadow rays walk the first inner child hit next (true: the nearest)
 constexpr int kMinLanes = 4;          // rays a warp takes at least when there are few
+constexpr int kIdle = -1, kNoRays = -2;  // instead of a lane's ray: waits for one; takes none
 constexpr int kMaxRounds = 1 << 22;   // per-warp round cap (~6k rounds per warp at 512x512)
 
 // COUNT: accumulate BVH nodes visited / primitives tested (and rays) into
@@ -139,7 +140,6 @@ __global__ void __launch_bounds__(128) persistent_trace_kernel(Src src, const __
   const SceneDev* sp = &s0;
   TraceCount tc{0, 0};
   uint32_t rays = 0;
-  int cur = -1;
   bool exhausted = false;
   int rounds = 0;
   // Fewer rays than lanes: spread over all warps instead of filling the first
@@ -149,13 +149,17 @@ __global__ void __launch_bounds__(128) persistent_trace_kernel(Src src, const __
   // 14.25 ms, 50,001 incoherent shadow rays 433 -> 370 us.  At least
   // kMinLanes = 4: 1 / 2 / 4 / 8 / 16 gave 4.62 / 4.77 / 4.85 / 5.03 / 5.14 ms
   // for two 256x192 frames and 634 / 626 / 612 / 607 / 621 us for 50,001 rays.
+  // (Lanes without rays are told apart by their cur: a mask of them kept through
+  // the loop took the shadow rays of a batch of scenes from 80 registers to 82,
+  // five blocks per SM instead of six, and 12 scenes' frames from 126.5 to 132.7
+  // ms.)
   const int per_warp = max(kMinLanes, min(32, (n + gridDim.x * 4 - 1) / (gridDim.x * 4)));
-  const unsigned lanes = FULL >> (32 - per_warp);
+  int cur = lane < per_warp ? kIdle : kNoRays;
   const int stragglers = (ANY_HIT ? kStragglersAnyHit : kStragglersClosest) * per_warp / 32;
   for (;;) {
     // refill idle lanes; a lane whose entry holds no ray (a shadow slot
     // left empty) fetches again at once instead of idling for a round
-    unsigned idle = __ballot_sync(FULL, cur < 0) & lanes;
+    unsigned idle = __ballot_sync(FULL, cur == kIdle);
     while (idle && !exhausted) {
       const int leader = __ffs(idle) - 1;
       const int want = __popc(idle);
@@ -163,9 +167,9 @@ __global__ void __launch_bounds__(128) persistent_trace_kernel(Src src, const __
       if (lane == leader) base = atomicAdd(fetch, want);
       base = __shfl_sync(FULL, base, leader);
       exhausted = base + want >= n;
-      if (cur < 0) {
+      if (cur == kIdle) {
         const int my = base + __popc(idle & ((1u << lane) - 1u));
-        if (((lanes >> lane) & 1u) && my < n) {
+        if (my < n) {
           f3 o, d;
           if (src.ray(my, &o, &d)) {
             if (MULTI) sp = &b.scenes[b.path_scene[src.path(my)]].s;
@@ -177,7 +181,7 @@ __global__ void __launch_bounds__(128) persistent_trace_kernel(Src src, const __
           }
         }
       }
-      idle = __ballot_sync(FULL, cur < 0) & lanes;
+      idle = __ballot_sync(FULL, cur == kIdle);
     }
     if (exhausted && __all_sync(FULL, cur < 0)) break;
     if (++rounds > kMaxRounds) {  // safety net: never spin on a logic error
@@ -206,7 +210,7 @@ __global__ void __launch_bounds__(128) persistent_trace_kernel(Src src, const __
       const bool done = trav_leaf<ANY_HIT, COUNT>(*sp, t, &tc);
       if (done || trav_finished(t)) {
         src.write(cur, t.h);
-        cur = -1;
+        cur = kIdle;
       }
     }
   }
