@@ -9,6 +9,7 @@
 // surviving paths (and therefore every result) does not depend on timing.
 #include <algorithm>
 #include <string>
+#include <type_traits>
 #include <vector>
 
 #include "hm_branch.h"
@@ -126,7 +127,10 @@ constexpr int kMaxRounds = 1 << 22;   // per-warp round cap (~6k rounds per warp
 // cnt[0..2] (an untimed instrumentation pass; timed frames use COUNT = false).
 // MULTI: the rays belong to the scenes of a batch (b.path_scene of the ray's
 // path selects the tree each lane walks).
-template <class Src, bool ANY_HIT, bool COUNT, bool MULTI>
+// SPREAD: few rays are spread over all warps (below).  Without it the kernel of
+// a caller's any-hit rays takes 80 registers instead of 93, six blocks per SM
+// instead of five; see hm_trace_rays.
+template <class Src, bool ANY_HIT, bool COUNT, bool MULTI, bool SPREAD = true>
 __global__ void __launch_bounds__(128) persistent_trace_kernel(Src src, const __grid_constant__ SceneDev s0,
                                                                Batch b, float tmin, float tmax,
                                                                int* __restrict__ fetch, int* err,
@@ -153,7 +157,7 @@ __global__ void __launch_bounds__(128) persistent_trace_kernel(Src src, const __
   // the loop took the shadow rays of a batch of scenes from 80 registers to 82,
   // five blocks per SM instead of six, and 12 scenes' frames from 126.5 to 132.7
   // ms.)
-  const int per_warp = max(kMinLanes, min(32, (n + gridDim.x * 4 - 1) / (gridDim.x * 4)));
+  const int per_warp = SPREAD ? max(kMinLanes, min(32, (n + gridDim.x * 4 - 1) / (gridDim.x * 4))) : 32;
   int cur = lane < per_warp ? kIdle : kNoRays;
   const int stragglers = (ANY_HIT ? kStragglersAnyHit : kStragglersClosest) * per_warp / 32;
   for (;;) {
@@ -221,7 +225,7 @@ __global__ void __launch_bounds__(128) persistent_trace_kernel(Src src, const __
   }
 }
 
-template <class Src, bool ANY_HIT>
+template <class Src, bool ANY_HIT, bool SPREAD = true>
 static int launch_persistent(const Src& src, const SceneDev& s, const Batch& b, float tmin, float tmax, int* fetch,
                              int* err, unsigned long long* cnt, bool counting, int max_blocks, cudaStream_t st) {
   // the traversal reads nodes with 32-byte loads (batch scenes: checked when the batch is built)
@@ -238,20 +242,20 @@ static int launch_persistent(const Src& src, const SceneDev& s, const Batch& b, 
       persistent_trace_kernel<Src, ANY_HIT, true, false><<<max_blocks, 128, 0, st>>>(src, s, b, tmin, tmax, fetch,
                                                                                      err, cnt);
     else
-      persistent_trace_kernel<Src, ANY_HIT, false, false><<<max_blocks, 128, 0, st>>>(src, s, b, tmin, tmax, fetch,
-                                                                                      err, cnt);
+      persistent_trace_kernel<Src, ANY_HIT, false, false, SPREAD><<<max_blocks, 128, 0, st>>>(
+          src, s, b, tmin, tmax, fetch, err, cnt);
   }
   HM_CHECK_LAUNCH("persistent_trace_kernel");
   return HM_OK;
 }
 
-template <class Src, bool ANY_HIT>
+template <class Src, bool ANY_HIT, bool SPREAD = true>
 static int persistent_blocks() {
   int dev = 0, sms = 152, per_sm = 4;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, persistent_trace_kernel<Src, ANY_HIT, false, false>, 128,
-                                                0);
+  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, persistent_trace_kernel<Src, ANY_HIT, false, false, SPREAD>,
+                                                128, 0);
   return sms * std::max(1, per_sm);
 }
 
@@ -1790,10 +1794,19 @@ extern "C" int hm_trace_rays(const hm_scene* h, const float* d_org, const float*
   cudaMemsetAsync(err, 0, 2 * sizeof(int), (cudaStream_t)stream);
   BatchRays src{d_org, d_dir, n, tmin, tmax, (float4*)d_hits};
   const Batch nob{nullptr, nullptr, 0};
-  int st = any_hit ? launch_persistent<BatchRays, true>(src, s->dev(), nob, tmin, tmax, err + 1, err, nullptr, false,
-                                                        persistent_blocks<BatchRays, true>(), (cudaStream_t)stream)
-                   : launch_persistent<BatchRays, false>(src, s->dev(), nob, tmin, tmax, err + 1, err, nullptr, false,
-                                                         persistent_blocks<BatchRays, false>(), (cudaStream_t)stream);
+  const auto launch = [&](auto any, auto spread) {
+    return launch_persistent<BatchRays, any(), spread()>(src, s->dev(), nob, tmin, tmax, err + 1, err, nullptr, false,
+                                                         persistent_blocks<BatchRays, any(), spread()>(),
+                                                         (cudaStream_t)stream);
+  };
+  // Five rays for each lane of the grid and more: there are none to spread, and
+  // six blocks per SM beat five.  Any-hit rays around straight / curly hair, us,
+  // spread and not: 300,007 449 / 802 and 456 / 827, 400,009 528 / 929 and 524 /
+  // 933, 500,009 612 / 1052 and 601 / 1049, 3,000,017 2511 / 4200 and 2355 / 3933.
+  const std::true_type yes;
+  const std::false_type no;
+  const bool spread = !any_hit || n < 5 * 128 * (int64_t)persistent_blocks<BatchRays, true>();
+  int st = !any_hit ? launch(no, yes) : spread ? launch(yes, yes) : launch(yes, no);
   if (st != HM_OK) {
     cudaFree(err);
     return st;
